@@ -203,6 +203,20 @@ decltype(auto) with_words(int W, F&& f) {
   }
 }
 
+// The same for the widths of the binned sweep, with the algebra.
+template <class F>
+decltype(auto) with_bins(int W, int alg, F&& f) {
+  auto by_alg = [&](auto w) {
+    return alg == 0 ? f(w, std::integral_constant<int, 0>{}) : f(w, std::integral_constant<int, 1>{});
+  };
+  switch (W) {
+    case 1: return by_alg(std::integral_constant<int, 1>{});
+    case 2: return by_alg(std::integral_constant<int, 2>{});
+    case 4: return by_alg(std::integral_constant<int, 4>{});
+    default: return by_alg(std::integral_constant<int, 8>{});
+  }
+}
+
 // Device resources of one propagation.  Slot 0 serves pq_run; a batch uses
 // slots 0..n-1.  Buffers grow on demand and are kept for the next run.
 struct Slot {
@@ -213,6 +227,7 @@ struct Slot {
   u64 bmask = ~3ULL;  // ~(slots per table bucket - 1) of the run the slot holds
   u64* status = nullptr;
   u64 cap = 0;
+  u64 seen_rows = 0;  // largest live count the slot's runs of width W reached
   int W = 0;
   int cur = 0;
   u32 epoch_base = 1;
@@ -244,6 +259,20 @@ struct Slot {
   double* host_factor = nullptr;
   unsigned char* host_keep = nullptr;
   size_t host_cap = 0;
+  // Binned sweep (pq_bins.cuh): two bin buffers of `room` rows, their spill
+  // tags, the counter sets, and the plan's windows.
+  u64* bin_keys[2] = {nullptr, nullptr};
+  double* bin_coeffs[2] = {nullptr, nullptr};
+  u32* bin_hash[2] = {nullptr, nullptr};
+  u32* spill_bin[2] = {nullptr, nullptr};
+  u64 room[2] = {0, 0};
+  int bin_W[2] = {0, 0};
+  u32* counts = nullptr;
+  pq::BinState* bin_state = nullptr;
+  pq::WinDesc* d_windows = nullptr;
+  size_t windows_cap = 0;
+  pq::BasisDesc* d_basis = nullptr;
+  size_t basis_cap = 0;
   int out_words = 0;  // width of out_keys (the caller's width)
   std::vector<u64> out_keys;
   std::vector<double> out_coeffs;
@@ -277,10 +306,28 @@ struct Slot {
     fam_table = fam_aux = nullptr;
     cls_cap = fam_cap = 0;
   }
+  void free_bins(int i) {
+    for (void* p : {(void*)bin_keys[i], (void*)bin_coeffs[i], (void*)bin_hash[i], (void*)spill_bin[i]})
+      if (p) dfree(p);
+    bin_keys[i] = nullptr;
+    bin_coeffs[i] = nullptr;
+    bin_hash[i] = spill_bin[i] = nullptr;
+    room[i] = 0;
+    bin_W[i] = 0;
+  }
   void free_all() {
     free_rows();
     free_ops();
     free_class();
+    free_bins(0);
+    free_bins(1);
+    for (void* p : {(void*)counts, (void*)bin_state, (void*)d_windows, (void*)d_basis})
+      if (p) dfree(p);
+    counts = nullptr;
+    bin_state = nullptr;
+    d_windows = nullptr;
+    d_basis = nullptr;
+    windows_cap = basis_cap = 0;
     for (void* p : {(void*)d_gates, (void*)d_tables, (void*)partials, (void*)frame_img, (void*)frame_sgn,
                     (void*)host_state, (void*)host_factor, (void*)host_keep})
       if (p) dfree(p);
@@ -367,6 +414,7 @@ struct pq_engine {
   // and per-op arrays, the segment checkpoints, and the pool size the last
   // default-sized gradient needed to record every op.
   DevBuf g_pool, g_lam, g_ops;
+  u32* d_lin = nullptr;  // linear hash tables of the binned sweep
   DevBuf sort_buf;  // radix-sort scratch and sorted rows (observable folding, sorted term output)
   std::vector<DevBuf> g_ck;
   size_t g_need = 0;
@@ -409,7 +457,7 @@ struct pq_engine {
     for (auto& s : slots) s.free_all();
     for (DevBuf* b : {&g_pool, &g_lam, &g_ops, &sort_buf}) b->release();
     for (DevBuf& b : g_ck) b.release();
-    for (void* p : {(void*)d_states, (void*)d_args, (void*)d_block_inst, (void*)d_err, (void*)d_idle})
+    for (void* p : {(void*)d_states, (void*)d_args, (void*)d_block_inst, (void*)d_err, (void*)d_idle, (void*)d_lin})
       if (p) dfree(p);
     for (void* p : {(void*)h_states, (void*)h_args, (void*)h_block_inst})
       if (p) cudaFreeHost(p);
@@ -477,8 +525,59 @@ struct pq_engine {
     S.cap = new_cap;
     S.tcap = ntcap;
     S.cur = 0;
+    if (S.W != Wn) S.seen_rows = 0;
     S.W = Wn;
     return rebuild_table(S, n);
+  }
+  // Room for `rows` dense rows of Wn words (both row buffers) without a hash
+  // table: what a binned run needs.  Keeps the first n rows of buffer S.cur.
+  int ensure_dense(Slot& S, u64 rows, u64 n, int Wn) {
+    if (S.W == Wn && S.cap >= rows) return PQ_OK;
+    u64* nk[2] = {nullptr, nullptr};
+    double* nc[2] = {nullptr, nullptr};
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+      e = dmalloc(&nk[i], rows * Wn * 8);
+      if (e == cudaSuccess) e = dmalloc(&nc[i], rows * 8);
+    }
+    if (e == cudaSuccess && n && S.keys[S.cur] && S.W == Wn) {
+      cudaMemcpyAsync(nk[S.cur], S.keys[S.cur], n * Wn * 8, cudaMemcpyDeviceToDevice, stream);
+      cudaMemcpyAsync(nc[S.cur], S.coeffs[S.cur], n * 8, cudaMemcpyDeviceToDevice, stream);
+      e = cudaStreamSynchronize(stream);
+    }
+    if (e != cudaSuccess) {
+      for (int i = 0; i < 2; ++i) {
+        if (nk[i]) dfree(nk[i]);
+        if (nc[i]) dfree(nc[i]);
+      }
+      return cuda_fail(e, "allocating term rows");
+    }
+    S.free_rows();
+    if (S.W != Wn) S.seen_rows = 0;
+    for (int i = 0; i < 2; ++i) {
+      S.keys[i] = nk[i];
+      S.coeffs[i] = nc[i];
+    }
+    S.cap = rows;
+    S.W = Wn;
+    return PQ_OK;
+  }
+  // A bin buffer of at least `rows` rows of Wn words; its contents are lost
+  // when it is replaced.
+  int ensure_bins(Slot& S, int i, u64 rows, int Wn) {
+    if (S.bin_W[i] == Wn && S.room[i] >= rows) return PQ_OK;
+    S.free_bins(i);
+    cudaError_t e;
+    if ((e = dmalloc(&S.bin_keys[i], rows * Wn * 8)) != cudaSuccess ||
+        (e = dmalloc(&S.bin_coeffs[i], rows * 8)) != cudaSuccess ||
+        (e = dmalloc(&S.bin_hash[i], rows * 4)) != cudaSuccess ||
+        (e = dmalloc(&S.spill_bin[i], rows / 8 * 4)) != cudaSuccess) {
+      S.free_bins(i);
+      return cuda_fail(e, "allocating bins");
+    }
+    S.room[i] = rows;
+    S.bin_W[i] = Wn;
+    return PQ_OK;
   }
   int rebuild_table(Slot& S, u64 n) {
     cudaMemsetAsync(S.table, 0xff, S.tcap * 8, stream);
@@ -590,6 +689,10 @@ struct Plan {
   // rows per thread of a many-row gate tile (0 = the kernel's 4), slots per
   // table bucket.
   u32 fuse_max = FUSE_DEFAULT, tile_items = 0, bucket_slots = BUCKET_DEFAULT;
+  bool binned = false;  // runs on the binned sweep (pq_bins.cuh)
+  u32 class_runs = 0;   // runs of Clifford rotations on disjoint units inside one window
+  std::vector<pq::WinDesc> windows;
+  std::vector<pq::BasisDesc> basis;
   bool fold_on_device = false;  // hk / hc hold the admitted terms unfolded (DEVICE_FOLD_MIN)
   std::vector<u64> hk;
   std::vector<double> hc;
@@ -722,6 +825,44 @@ int prepare(pq_engine* E, Plan& P, const Inputs& in, int W) {
   return PQ_OK;
 }
 
+// The binned sweep's linear hash: eight byte tables of random words
+// (splitmix64), the same ones on the host and the device; word w's lookup is
+// rotated by 5 w bits.  XOR of keys is XOR of hashes.
+const std::vector<u32>& lin_table() {
+  static const std::vector<u32> t = [] {
+    std::vector<u32> v(pq::LIN_WORDS, 0);
+    u64 x = 0x1234567890abcdefULL;
+    auto next = [&] {
+      x += 0x9E3779B97F4A7C15ULL;
+      u64 z = x;
+      z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+      z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+      return (u32)((z ^ (z >> 31)) >> 16);
+    };
+    for (int b = 0; b < 8; ++b) {
+      u32 bit[8];
+      for (u32& w : bit) w = next();
+      for (u32 i = 0; i < 256; ++i)
+        for (int j = 0; j < 8; ++j)
+          if (i >> j & 1) v[256 * b + i] ^= bit[j];
+    }
+    return v;
+  }();
+  return t;
+}
+u32 lin_hash(const u64* k, int W) {
+  const std::vector<u32>& t = lin_table();
+  u32 h = 0;
+  for (int w = 0; w < W; ++w) {
+    if (!k[w]) continue;
+    u32 x = 0;
+    for (int b = 0; b < 8; ++b) x ^= t[256 * b + (k[w] >> (8 * b) & 255)];
+    const int r = (5 * w) & 31;
+    h ^= r ? (x << r) | (x >> (32 - r)) : x;
+  }
+  return h;
+}
+
 // Sizes the slot's buffers for the plan, uploads the admitted rows and noise
 // tables, rebuilds the table.
 int setup_slot(pq_engine* E, Slot& S, Plan& P) {
@@ -729,8 +870,14 @@ int setup_slot(pq_engine* E, Slot& S, Plan& P) {
   const int W = P.W;
   S.bmask = ~(u64)(P.bucket_slots - 1);
   const u64 want_cap = next_pow2(std::max<u64>(4 * P.n0, 1ULL << 16));
-  if (S.W != W || S.cap < want_cap) {
-    if (int rc = E->resize(S, std::max(want_cap, S.W == W ? S.cap : 0), 0, S.cur, W)) return rc;
+  if (P.binned) {
+    if (int rc = E->ensure_dense(S, std::max(want_cap, S.W == W ? S.cap : 0), 0, W)) return rc;
+  } else if (S.W != W || S.cap < want_cap || S.tcap != 2 * S.cap) {
+    // as large as the row sweep needed for the slot's largest run so far
+    const u64 seen = S.W == W ? std::max(S.cap, std::min(next_pow2(4 * S.seen_rows), E->row_ceiling())) : 0;
+    int rc = E->resize(S, std::max(want_cap, seen), 0, S.cur, W);
+    if (rc == PQ_ERR_OOM && seen > want_cap) rc = E->resize(S, want_cap, 0, S.cur, W);
+    if (rc) return rc;
   }
   S.cur = 0;
   if (P.n0 && P.fold_on_device) {
@@ -759,7 +906,8 @@ int setup_slot(pq_engine* E, Slot& S, Plan& P) {
     cudaMemcpyAsync(S.keys[0], P.hk.data(), P.n0 * W * 8, cudaMemcpyHostToDevice, E->stream);
     cudaMemcpyAsync(S.coeffs[0], P.hc.data(), P.n0 * 8, cudaMemcpyHostToDevice, E->stream);
   }
-  if (int rc = E->rebuild_table(S, P.n0)) return rc;
+  if (!P.binned)
+    if (int rc = E->rebuild_table(S, P.n0)) return rc;
   const size_t n_ops_max = P.in->n_gates + P.in->n_layers + 1;
   if (int rc = E->ensure_ops(S, n_ops_max)) return rc;
   const size_t gbytes = std::max<size_t>(P.in->n_gates, 1) * gdesc_words(W) * 8;
@@ -834,7 +982,7 @@ int build_ops(Plan& P, NeedN need_n) {
         gd.sn = sn;
         gd.cs = cs;
         gd.pivot = 0;
-        gd.pad_ = 0;
+        gd.hash = lin_hash(gc.data(), W);
         const size_t off = P.gdesc.size();
         P.gdesc.resize(off + sizeof gd / 8);
         std::memcpy(&P.gdesc[off], &gd, sizeof gd);
@@ -1071,6 +1219,125 @@ pq::SweepArgs sweep_args(Slot& S, const Plan& P, pq::SweepState* st, u32 blk_beg
   return a;
 }
 
+// Which runs take the binned sweep.  Left on the row sweep: rules that need
+// the whole live set between rotations (a TermBudget floor, plugins asked per
+// row), the per-rotation log, keys over 8 words (too few rows fit a block),
+// and runs that set the row sweep's own parameters (a fixed grid, its tuning
+// knobs, a row or memory limit or a look-back limit on the engine), which ask
+// for that sweep's behaviour.
+bool use_bins(const pq_engine* E, const Plan& P) {
+  const pq_run_config* c = P.in->cfg;
+  if (P.has_floor || P.host_ops || P.log || P.W > 8) return false;
+  if (c->blocks_per_sm || c->fuse_max || c->tile_items || c->bucket_slots) return false;
+  return !E->lim.max_rows && !E->lim.max_device_bytes && !E->lim.lookback_spins;
+}
+
+// Cuts the op sequence into windows (pq_bins.cuh).  From each rotation on the
+// longer of two runs is taken: a span window, as long as the rank of its
+// generators stays within bin_rank, or -- Pauli generators on pairwise
+// disjoint qubits under a weight cut of at most bin_rank -- a disjoint
+// window.  Noise ends a window and is part of it.
+void plan_windows(Plan& P) {
+  const int W = P.W;
+  const size_t gw = gdesc_words(W), no = P.ops.size();
+  const u32 rank_max = pq::bin_rank(W);
+  auto is_rot = [&](size_t i) { return P.ops[i].kind == pq::OP_GATE || P.ops[i].kind == pq::OP_PHASE; };
+  auto gen = [&](size_t i) { return &P.gdesc[P.ops[i].idx * gw]; };
+  auto lowest = [&](const u64* g) {
+    for (int w = 0; w < W; ++w)
+      if (g[w]) return (int)(64 * w + __builtin_ctzll(g[w]));
+    return -1;
+  };
+  auto bit = [](const u64* g, int b) { return (g[b >> 6] >> (b & 63)) & 1; };
+  const bool disjoint_ok = P.alg == 0 && P.has_w && P.wcut <= rank_max;
+  std::vector<std::vector<u64>> span;
+  std::vector<int> pivot;
+  std::vector<u64> used(W), g(W);
+  for (size_t i = 0; i < no;) {
+    pq::WinDesc w{};
+    w.op = (u32)i;
+    w.basis = (u32)P.basis.size();
+    size_t len = 0;
+    if (is_rot(i)) {
+      span.clear();
+      pivot.clear();
+      size_t la = 0;
+      for (; i + la < no && la < pq::WIN_MAX && is_rot(i + la); ++la) {
+        if (P.ops[i + la].kind == pq::OP_PHASE) continue;
+        std::copy(gen(i + la), gen(i + la) + W, g.begin());
+        for (size_t b = 0; b < span.size(); ++b)
+          if (bit(g.data(), pivot[b]))
+            for (int x = 0; x < W; ++x) g[x] ^= span[b][x];
+        const int pv = lowest(g.data());
+        if (pv < 0) continue;
+        if (span.size() >= rank_max) break;
+        for (auto& v : span)
+          if (bit(v.data(), pv))
+            for (int x = 0; x < W; ++x) v[x] ^= g[x];
+        span.push_back(g);
+        pivot.push_back(pv);
+      }
+      size_t lb = 0;
+      if (disjoint_ok) {
+        std::fill(used.begin(), used.end(), 0);
+        for (; i + lb < no && lb < pq::WIN_MAX && is_rot(i + lb); ++lb) {
+          if (P.ops[i + lb].kind == pq::OP_PHASE) continue;
+          const u64* v = gen(i + lb);
+          bool clash = false;
+          for (int x = 0; x < W; ++x) clash |= ((v[x] | (v[x] >> 1)) & EVEN & used[x]) != 0;
+          if (clash) break;
+          for (int x = 0; x < W; ++x) used[x] |= (v[x] | (v[x] >> 1)) & EVEN;
+        }
+      }
+      if (lb > la) {
+        len = lb;
+        w.disjoint = 1;
+        for (size_t k = 0; k < len; ++k) {
+          const int pv = lowest(gen(i + k));
+          if (P.ops[i + k].kind != pq::OP_PHASE && pv >= 0)
+            P.basis.push_back({(u32)pv, lin_hash(gen(i + k), W), (u32)k, 0});
+        }
+      } else {
+        len = la;
+        for (size_t b = 0; b < span.size(); ++b)
+          P.basis.push_back({(u32)pivot[b], lin_hash(span[b].data(), W), 0, 0});
+      }
+      w.gate = P.ops[i].idx;
+      w.n_gates = (u32)len;
+      i += len;
+    }
+    w.n_basis = (u32)P.basis.size() - w.basis;
+    if (disjoint_ok && P.wcut <= pq::CLASS_KMAX) {  // runs of Clifford rotations on disjoint qubits (pq_result::class_ops)
+      size_t run = 0;
+      for (size_t k = w.op; k < i; ++k) {
+        const u64* v = gen(k);
+        double cs = 0;
+        with_words(W, [&](auto ww) {
+          pq::GateDesc<decltype(ww)::value> gd;
+          std::memcpy(&gd, v, sizeof gd);
+          cs = gd.cs;
+          return 0;
+        });
+        const bool clifford = P.ops[k].kind == pq::OP_GATE && std::fabs(cs) < EPS_CLASSIFY && lowest(v) >= 0;
+        bool clash = false;
+        for (int x = 0; x < W; ++x) clash |= run && ((v[x] | (v[x] >> 1)) & EVEN & used[x]) != 0;
+        if (!clifford || clash) run = 0;
+        if (!clifford) continue;
+        if (!run) std::fill(used.begin(), used.end(), 0);
+        for (int x = 0; x < W; ++x) used[x] |= (v[x] | (v[x] >> 1)) & EVEN;
+        if (++run == CLASS_MIN) ++P.class_runs;
+      }
+    }
+    if (i < no && !is_rot(i)) {
+      w.noise = P.ops[i].kind == pq::OP_NOISE_COMPACT ? 2 : 1;
+      w.table = P.ops[i].idx;
+      ++i;
+    }
+    w.op_end = (u32)i;
+    P.windows.push_back(w);
+  }
+}
+
 pq::SweepState fresh_state(const pq_engine* E, const Plan& P) {
   pq::SweepState s{};
   E->init_waits(s);
@@ -1196,6 +1463,148 @@ int execute_launches(pq_engine* E, Slot& S, Plan& P, int grid, bool* began, size
     if (int rc = absorb_state(E, S, P, E->h_states[0])) return rc;
   }
   return PQ_OK;
+}
+
+// Runs every op of a plan on the binned sweep: one block alone while the rows
+// fit it, then the windows on the whole grid; a buffer that turned out too
+// small is grown and the sweep goes on from the window that needed it.
+int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
+  cudaError_t e;
+  const int W = P.W;
+  const size_t no = P.ops.size();
+  constexpr u64 ROOM = 1ULL << 20;  // rows of a bin buffer to begin with
+  if (!E->d_lin) {
+    if ((e = dmalloc(&E->d_lin, pq::LIN_WORDS * 4)) != cudaSuccess) return E->cuda_fail(e, "hash tables");
+    cudaMemcpyAsync(E->d_lin, lin_table().data(), pq::LIN_WORDS * 4, cudaMemcpyHostToDevice, E->stream);
+  }
+  if (!S.counts && (e = dmalloc(&S.counts, 3 * (size_t)pq::COUNT_WORDS * 4)) != cudaSuccess)
+    return E->cuda_fail(e, "bin counters");
+  if (!S.bin_state && (e = dmalloc(&S.bin_state, sizeof(pq::BinState))) != cudaSuccess)
+    return E->cuda_fail(e, "bin state");
+  if ((e = grow_pair<pq::WinDesc>(&S.d_windows, nullptr, &S.windows_cap, std::max<size_t>(P.windows.size(), 1))) !=
+          cudaSuccess ||
+      (e = grow_pair<pq::BasisDesc>(&S.d_basis, nullptr, &S.basis_cap, std::max<size_t>(P.basis.size(), 1))) !=
+          cudaSuccess)
+    return E->cuda_fail(e, "windows");
+  for (int i = 0; i < 2; ++i)
+    if (int rc = E->ensure_bins(S, i, std::max(ROOM, S.bin_W[i] == W ? S.room[i] : 0), W)) return rc;
+  upload_ops(E, S, P);
+  if (no) {
+    cudaMemcpyAsync(S.d_windows, P.windows.data(), P.windows.size() * sizeof(pq::WinDesc), cudaMemcpyHostToDevice,
+                    E->stream);
+    if (!P.basis.empty())
+      cudaMemcpyAsync(S.d_basis, P.basis.data(), P.basis.size() * sizeof(pq::BasisDesc), cudaMemcpyHostToDevice,
+                      E->stream);
+    cudaMemsetAsync(S.tickets, 0, no * 4, E->stream);
+    cudaMemsetAsync(S.stamps, 0, no * 8, E->stream);
+  }
+  cudaMemsetAsync(S.counts, 0, 3 * (size_t)pq::COUNT_WORDS * 4, E->stream);
+  cudaMemsetAsync(S.bin_state, 0, sizeof(pq::BinState), E->stream);
+  pq::BinArgs a{};
+  a.ops = S.d_ops;
+  a.gates = S.d_gates;
+  a.windows = S.d_windows;
+  a.basis = S.d_basis;
+  a.tables = S.d_tables;
+  a.lin = E->d_lin;
+  a.n_gdesc = (u32)(P.gdesc.size() / gdesc_words(W));
+  a.n_windows = (u32)P.windows.size();
+  a.table_len = (u32)P.tlen;
+  a.n_units = P.n_units;
+  a.op_begin = 0;
+  a.op_end = (u32)no;
+  a.max_weight = P.wcut;
+  a.has_min_coeff = P.has_c;
+  a.min_coeff = P.ccut;
+  a.n0 = P.n0;
+  a.counts = S.counts;
+  a.count_words = pq::COUNT_WORDS;
+  a.born = S.tickets;
+  a.anti = S.anti;
+  a.hist = S.hist;
+  a.stamps = S.stamps;
+  a.st = E->d_states;
+  a.bs = S.bin_state;
+  a.hold_block = E->lim.hold_block;
+  a.hold_us = std::min<u32>(E->lim.hold_us, 100000);
+  const int grid = with_bins(W, P.alg, [](auto w, auto alg) { return pq::bins_grid<w, alg>(); });
+  if (grid <= 0) return E->fail(PQ_ERR_CUDA, "the binned sweep does not fit this device");
+  pq::BinState hb{};
+  for (bool first = true;; first = false) {
+    for (int i = 0; i < 2; ++i) {
+      a.bin_keys[i] = S.bin_keys[i];
+      a.bin_coeffs[i] = S.bin_coeffs[i];
+      a.bin_hash[i] = S.bin_hash[i];
+      a.spill_bin[i] = S.spill_bin[i];
+      a.room[i] = S.room[i];
+    }
+    a.keys = S.keys[S.cur];
+    a.coeffs = S.coeffs[S.cur];
+    a.dense_room = S.cap;
+    if (first) {
+      E->h_states[0] = fresh_state(E, P);
+      cudaMemcpyAsync(E->d_states, E->h_states, sizeof(pq::SweepState), cudaMemcpyHostToDevice, E->stream);
+    }
+    if (!*began) {
+      cudaEventRecord(E->ev_begin, E->stream);
+      *began = true;
+    }
+    cudaEventRecord(E->ev_l0, E->stream);
+    if (first) {
+      ++E->launches;
+      ++P.sweep_launches;
+      e = with_bins(W, P.alg, [&](auto w, auto alg) { return pq::launch_solo<w, alg>(a, E->stream); });
+      if (e != cudaSuccess) return E->cuda_fail(e, "solo launch");
+    }
+    ++E->launches;
+    ++P.sweep_launches;
+    e = with_bins(W, P.alg, [&](auto w, auto alg) { return pq::launch_bins<w, alg>(a, grid, E->stream); });
+    if (e != cudaSuccess) return E->cuda_fail(e, "binned sweep launch");
+    cudaEventRecord(E->ev_l1, E->stream);
+    cudaMemcpyAsync(E->h_states, E->d_states, sizeof(pq::SweepState), cudaMemcpyDeviceToHost, E->stream);
+    cudaMemcpyAsync(&hb, S.bin_state, sizeof hb, cudaMemcpyDeviceToHost, E->stream);
+    if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "binned sweep");
+    float ms = 0;
+    cudaEventElapsedTime(&ms, E->ev_l0, E->ev_l1);
+    P.sweep_ms += ms;
+    const pq::SweepState& h = E->h_states[0];
+    if (h.error & pq::ERR_BARRIER_TIMEOUT)
+      return E->fail(PQ_ERR_DEVICE_TIMEOUT, "a grid barrier wait expired on the device");
+    if (h.error) return E->fail(PQ_ERR_CUDA, "device reported error bits " + std::to_string(h.error));
+    if (!hb.stopped) {
+      P.n_live = h.n[0];
+      P.done = no;
+      return PQ_OK;
+    }
+    // The buffer the stopped window was filling (or the dense rows) is grown.
+    const u32 fill = hb.dense_start ? 0 : hb.phase + 1;
+    if (!hb.dense_start && P.windows.back().op_end > hb.op && P.windows.back().op <= hb.op) {
+      if (int rc = E->ensure_dense(S, next_pow2(std::max<u64>(hb.n_dense, S.cap + 1)), 0, W)) return rc;
+    } else {
+      const u64 want = std::max<u64>(4 * S.room[fill & 1], next_pow2(4 * hb.rows));
+      if (int rc = E->ensure_bins(S, (int)(fill & 1), want, W)) return rc;
+    }
+    // Everything the stopped window counted is dropped.
+    for (u32 s = 0; s < 3; ++s) {
+      if (!hb.dense_start && s == hb.phase % 3) continue;
+      cudaMemsetAsync(S.counts + (size_t)s * pq::COUNT_WORDS, 0, (size_t)pq::COUNT_WORDS * 4, E->stream);
+      hb.n_spill[s] = 0;
+    }
+    for (u32 s = 0; s < 3; ++s) {
+      hb.n[s] = hb.grown[s] = 0;
+      hb.ticket[s] = hb.fail[s] = 0;
+    }
+    hb.stopped = 0;
+    hb.n_dense = 0;
+    a.resume = hb.dense_start ? 0 : 1;
+    a.phase0 = hb.dense_start ? 0 : hb.phase;
+    if (no > hb.op) {
+      cudaMemsetAsync(S.tickets + hb.op, 0, (no - hb.op) * 4, E->stream);
+      cudaMemsetAsync(S.anti + hb.op, 0, (no - hb.op) * 8, E->stream);
+    }
+    cudaMemcpyAsync(S.bin_state, &hb, sizeof hb, cudaMemcpyHostToDevice, E->stream);
+    if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "binned sweep");
+  }
 }
 
 // True if op k needs decisions from a plugin on the host: every rotation when
@@ -1426,7 +1835,7 @@ int finalize(pq_engine* E, Slot& S, Plan& P, std::vector<pq::ExpectPartial>* par
     }
     const u64* out_k = S.keys[src];
     const double* out_c = S.coeffs[src];
-    if (in.cfg->want_terms == 2) {  // in key order: the radix sort into the engine's sort buffer
+    if (in.cfg->want_terms == 2 || P.binned) {  // in key order (bins hold rows in no fixed order): the radix sort into the engine's sort buffer
       const u64 sw = pq::sort_scratch_words(n_fin, W);
       if ((e = E->sort_buf.ensure((sw + n_fin * (u64)(W + 1)) * 8)) != cudaSuccess)
         return E->cuda_fail(e, "sort scratch");
@@ -1482,7 +1891,26 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
     cudaMemcpyAsync(hist.data(), S.hist, no * 8, cudaMemcpyDeviceToHost, E->stream);
     cudaMemcpyAsync(anti.data(), S.anti, no * 8, cudaMemcpyDeviceToHost, E->stream);
     cudaMemcpyAsync(stamps.data(), S.stamps, no * 8, cudaMemcpyDeviceToHost, E->stream);
+    std::vector<u32> born(P.binned ? no : 0);
+    if (P.binned) cudaMemcpyAsync(born.data(), S.tickets, no * 4, cudaMemcpyDeviceToHost, E->stream);
     if (cudaError_t e = cudaStreamSynchronize(E->stream)) return E->cuda_fail(e, "op statistics");
+    if (P.binned) {  // live counts from the rows each rotation created; one stamp per window
+      u64 n = P.n0;
+      for (size_t i = 0; i < no; ++i) {
+        const u32 kind = P.ops[i].kind;
+        if (kind == pq::OP_GATE && 2 * n > MAX_ROWS)
+          return E->fail(PQ_ERR_CEILING, "term index ceiling reached: " + std::to_string(2 * n) +
+                                             " rows would exceed the engine's capacity");
+        if (kind == pq::OP_NOISE_COMPACT)
+          n = hist[i];
+        else if (kind != pq::OP_NOISE_SCALE)
+          n += born[i];
+        hist[i] = n;
+        P.peak = std::max(P.peak, n);
+      }
+      for (size_t i = no; i-- > 0;)
+        if (!stamps[i] && i + 1 < no) stamps[i] = stamps[i + 1];
+    }
   }
   if (in.n_terms_out)
     for (size_t g = 0; g < in.n_gates; ++g) in.n_terms_out[g] = P.gate_op[g] >= 0 ? hist[P.gate_op[g]] : P.n0;
@@ -1544,21 +1972,24 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
         res->sum_kept += P.ops[i].kind == pq::OP_NOISE_COMPACT ? hist[i] : 0;
     }
   }
+  res->class_ops += P.class_runs;
   res->sweep_ms = P.sweep_ms;
   res->sweep_launches = P.sweep_launches;
   res->n_final = P.n_live;
   res->peak_terms = P.peak;
+  S.seen_rows = std::max(S.seen_rows, P.peak);
   res->sparse_key_bytes = P.n_live * P.W * 8 + S.tcap * 8;
   res->n_layers_run = in.n_layers;
   res->n_gates_run = in.n_gates;
   return PQ_OK;
 }
 
-int run_one(pq_engine* E, const Inputs& in, int W) {
+int run_one(pq_engine* E, const Inputs& in, int W, bool bins = true) {
   if (int rc = E->ensure_slots(1)) return rc;
   Slot& S = E->slots[0];
   Plan P;
   if (int rc = prepare(E, P, in, W)) return rc;
+  P.binned = bins && use_bins(E, P);
   if (int rc = setup_slot(E, S, P)) return rc;
   const int grid = with_words(W, [&](auto w) {
     constexpr int WW = decltype(w)::value;
@@ -1572,9 +2003,21 @@ int run_one(pq_engine* E, const Inputs& in, int W) {
     return PQ_OK;
   };
   if (int rc = build_ops(P, need_n)) return rc;
-  fuse_classes(P);
-  fuse_groups(P);
-  if (int rc = execute_single(E, S, P, grid, &began)) return rc;
+  if (P.binned) {
+    plan_windows(P);
+    const int rc = execute_bins(E, S, P, &began);
+    if (rc == PQ_ERR_OOM) {  // the row sweep may still fit
+      S.free_bins(0);
+      S.free_bins(1);
+      S.free_rows();
+      return run_one(E, in, W, false);
+    }
+    if (rc) return rc;
+  } else {
+    fuse_classes(P);
+    fuse_groups(P);
+    if (int rc = execute_single(E, S, P, grid, &began)) return rc;
+  }
   if (!began) cudaEventRecord(E->ev_begin, E->stream);
   std::vector<pq::ExpectPartial> parts;
   if (int rc = finalize(E, S, P, &parts)) return rc;

@@ -1068,6 +1068,19 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Failure tests only: a bounded hold, so the others' waits on this block expire.
+__device__ __noinline__ void hold(u32 us) {
+  u64 t0, t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (u32 i = 0; i < (1u << 20); ++i) {  // the host caps the hold at 100 ms
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    if (t - t0 >= (u64)us * 1000ull) break;
+    __nanosleep(1000);
+  }
+}
+
+#include "pq_bins.cuh"
+
 template <int W, int ALG>
 __device__ __forceinline__ void sweep_body(const SweepArgs& a, const Grp grp) {
   __shared__ TileSmem sm;
@@ -1124,16 +1137,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a, const Grp grp) {
   // live counts, so the offsets agree without communication.
   u64 rb = a.rec_idx ? ld_volatile(&st->rec_next) : 0, rkb = a.rec_idx ? ld_volatile(&st->rec_key_next) : 0;
   bool rec_on = a.rec_idx && !*(volatile u32*)&st->rec_full;
-  if (a.hold_us && grp.bid == a.hold_block && threadIdx.x == 0) {
-    // failure tests only: a bounded hold, so the others' waits on this block expire
-    u64 t0, t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    for (u32 i = 0; i < (1u << 20); ++i) {  // the host caps hold_us at 100 ms
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      if (t - t0 >= (u64)a.hold_us * 1000ull) break;
-      __nanosleep(1000);
-    }
-  }
+  if (a.hold_us && grp.bid == a.hold_block && threadIdx.x == 0) hold(a.hold_us);
   __syncthreads();
   bool stopped = false;  // a capacity stop inside a fused op
   while (op < a.op_end) {
@@ -1357,6 +1361,35 @@ __global__ void __launch_bounds__(BLOCK, 6) sweep_kernel_occ(const SweepArgs a) 
 template <int W, int ALG>
 __global__ void __launch_bounds__(BLOCK, 2) sweep_kernel_two(const SweepArgs a) {
   sweep_body<W, ALG>(a, Grp{blockIdx.x, gridDim.x});
+}
+
+// The binned sweep (pq_bins.cuh) for keys of at most 8 words.  Rows a block
+// holds: two blocks per SM on the grid, one block with a whole SM's shared
+// memory solo.  256 threads: every warp issues a rotation's fixed part
+// (barriers, descriptor, counts), so more warps cost more than their rows
+// give -- 512 threads (64 registers, spilling) ran kicked Ising 10x10 in 9.5
+// ms against 7.4 and the 24-site Givens circuit in 14.0 against 14.1 ms; three
+// blocks per SM of 2,304 rows took the latter from 13.3 to 17.2 ms (fuller
+// bins, more of them split).
+template <int W>
+struct BinSize {
+  static constexpr int T = 256;
+  static constexpr int BLOCKS = 2;  // per SM
+  static constexpr int GRID_R = W == 1 ? 3328 : (W == 2 ? 2560 : (W == 4 ? 2048 : 1152));
+  static constexpr int SOLO_R = W == 1 ? 7168 : 2 * GRID_R;
+  using Grid = BinSmem<W, T, GRID_R, (W <= 2 ? 8192 : 4096)>;
+  using Solo = BinSmem<W, T, SOLO_R, (W <= 2 ? 16384 : 8192)>;
+};
+
+template <int W, int ALG>
+__global__ void __launch_bounds__(BinSize<W>::T, 1) solo_kernel(const BinArgs a) {
+  extern __shared__ __align__(16) unsigned char bin_smem[];
+  solo_body<W, ALG>(a, *reinterpret_cast<typename BinSize<W>::Solo*>(bin_smem));
+}
+template <int W, int ALG>
+__global__ void __launch_bounds__(BinSize<W>::T, BinSize<W>::BLOCKS) bins_kernel(const BinArgs a) {
+  extern __shared__ __align__(16) unsigned char bin_smem[];
+  bins_body<W, ALG>(a, Grp{blockIdx.x, gridDim.x}, *reinterpret_cast<typename BinSize<W>::Grid*>(bin_smem));
 }
 
 // A batch: each instance owns the contiguous blocks [blk_begin, blk_begin +
@@ -1761,6 +1794,39 @@ cudaError_t launch_sweep(const SweepArgs& a, int grid, cudaStream_t s, int build
 }
 
 template <int W, int ALG>
+cudaError_t launch_solo(const BinArgs& a, cudaStream_t s) {
+  using S = typename BinSize<W>::Solo;
+  static_assert(sizeof(S) <= 227 * 1024, "solo shared memory");
+  if (cudaError_t e = cudaFuncSetAttribute(solo_kernel<W, ALG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(S)))
+    return e;
+  solo_kernel<W, ALG><<<1, S::T, sizeof(S), s>>>(a);
+  return cudaGetLastError();
+}
+
+template <int W, int ALG>
+int bins_grid() {
+  using S = typename BinSize<W>::Grid;
+  static_assert(BinSize<W>::BLOCKS * (sizeof(S) + 1024) <= 228 * 1024, "resident blocks");
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaFuncSetAttribute(bins_kernel<W, ALG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(S)) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bins_kernel<W, ALG>, S::T, sizeof(S)) != cudaSuccess)
+    return 0;
+  return sms * per;
+}
+
+template <int W, int ALG>
+cudaError_t launch_bins(const BinArgs& a, int grid, cudaStream_t s) {
+  using S = typename BinSize<W>::Grid;
+  BinArgs args = a;
+  void* params[] = {&args};
+  return cudaLaunchCooperativeKernel((const void*)bins_kernel<W, ALG>, dim3(grid), dim3(S::T), params, sizeof(S), s);
+}
+
+template <int W, int ALG>
 cudaError_t launch_batch_sweep(const SweepArgs* args, const u32* block_inst, int grid, cudaStream_t s) {
   void* params[] = {(void*)&args, (void*)&block_inst};
   return cudaLaunchCooperativeKernel((const void*)batch_sweep_kernel<W, ALG>, dim3(grid), dim3(BLOCK), params, 0,
@@ -1838,6 +1904,10 @@ cudaError_t launch_conjugate(const u64* keys, const double* coeffs, u64 n, const
   template int adjoint_grid<Wv, Av>();                                                                  \
   template cudaError_t launch_expect<Wv, Av>(const ExpectArgs&, const u64*, const double*, u64,         \
                                              ExpectPartial*, int, cudaStream_t);
+#define PQ_INSTANTIATE_BINS(Wv, Av)                                                                     \
+  template int bins_grid<Wv, Av>();                                                                     \
+  template cudaError_t launch_solo<Wv, Av>(const BinArgs&, cudaStream_t);                               \
+  template cudaError_t launch_bins<Wv, Av>(const BinArgs&, int, cudaStream_t);
 #define PQ_INSTANTIATE_KEYS(Wv)                                                                         \
   template cudaError_t launch_rebuild<Wv>(const u64*, u64, u64*, u64, u64, u32*, cudaStream_t);         \
   template cudaError_t launch_conjugate<Wv>(const u64*, const double*, u64, const u64*, const int*, u32, int, \
@@ -1860,9 +1930,17 @@ PQ_INSTANTIATE_KEYS(PQ_ONLY_WIDTH)
 #endif
 #elif defined(PQ_ONLY_WIDTH)
 PQ_INSTANTIATE_W(PQ_ONLY_WIDTH)
+#if PQ_ONLY_WIDTH <= 8
+PQ_INSTANTIATE_BINS(PQ_ONLY_WIDTH, 0)
+PQ_INSTANTIATE_BINS(PQ_ONLY_WIDTH, 1)
+#endif
 #else
 PQ_INSTANTIATE_W(1)
 PQ_INSTANTIATE_W(2)
+PQ_INSTANTIATE_BINS(1, 0)
+PQ_INSTANTIATE_BINS(1, 1)
+PQ_INSTANTIATE_BINS(2, 0)
+PQ_INSTANTIATE_BINS(2, 1)
 #endif
 
 }  // namespace pq

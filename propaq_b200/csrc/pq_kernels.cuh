@@ -47,7 +47,7 @@ struct GateDesc {
   double sn, cs;  // sin(angle), cos(angle) from the host libm
   u32 pivot;      // in a class: a key bit of this generator that no other
                   // generator of the class has (its family coordinate)
-  u32 pad_;
+  u32 hash;       // binned sweep: the generator's linear hash (lin_table)
 };
 
 // Device-resident state of a sweep, one per engine.
@@ -151,6 +151,91 @@ struct SweepArgs {
   u32 tile_items;
   u32 pad1_;
 };
+
+// ------------------------------------------------------------ binned sweep
+// See pq_bins.cuh.
+constexpr u32 WIN_MAX = 128;       // rotations of one window
+constexpr u32 BIN_MAX = 1u << 18;  // bins of one buffer
+constexpr u32 COUNT_WORDS = BIN_MAX;  // words of one counter set (fewer bins, wider stride: choose_layout)
+constexpr u32 LIN_WORDS = 8 * 256;  // linear hash: 8 byte tables
+// Largest rank of a span window / family dimension of a disjoint window: a
+// group of 2^rank rows must fit the rows a block holds.
+__host__ __device__ constexpr u32 bin_rank(int W) { return W <= 4 ? 11u : 10u; }
+
+// A window: rotations [op, op + n_gates), then the noise op at op + n_gates
+// if there is one (op_end is past it).
+struct WinDesc {
+  u32 op, op_end;
+  u32 n_gates, gate;   // rotations; descriptor of the first
+  u32 noise, table;    // 0 none, 1 scale, 2 scale and reclaim; its noise table
+  u32 basis, n_basis;  // grouping: BasisDescs
+  u32 disjoint;        // a basis vector counts only where its rotation anticommutes
+};
+struct BasisDesc {
+  u32 bit;   // pivot key bit, in no other vector of the window's basis
+  u32 hash;  // linear hash of the vector
+  u32 gate;  // disjoint windows: the rotation, counted from the window's first
+  u32 pad_;
+};
+
+// Device state of a binned sweep; the sets are indexed by window count mod 3.
+struct BinState {
+  u64 n[3];        // rows in the set's bins
+  u64 grown[3];    // rows created by the window that filled it
+  u64 n_dense;     // rows written dense at the end
+  u32 n_spill[3];  // rows past a full bin
+  u32 ticket[3];   // bins handed out
+  u32 fail[3];     // the set's buffer was too small
+  // Where a sweep stopped for a buffer the host has to grow.
+  u32 stopped, dense_start;  // dense_start: before any row was dealt
+  u32 op, phase;   // first op not run; count of buffer fills so far
+  u64 rows;
+  u32 bins, stride, cap;
+  float rho;
+};
+
+struct BinArgs {
+  const OpDesc* ops;
+  const void* gates;  // GateDesc<W>[], in op order
+  const WinDesc* windows;
+  const BasisDesc* basis;
+  const double* tables;
+  const u32* lin;     // linear hash tables
+  u32 n_gdesc, n_windows;
+  u32 table_len, n_units;
+  u32 op_begin, op_end;
+  u32 first_gate, pad_;  // gate descriptor of the first rotation from op_begin on
+  u32 max_weight, has_min_coeff;
+  double min_coeff;
+  u64 n0;             // dense rows at entry
+  u64* keys;          // dense rows: the input and the result
+  double* coeffs;
+  u64 dense_room;
+  u64* bin_keys[2];
+  double* bin_coeffs[2];
+  u32* bin_hash[2];
+  u32* spill_bin[2];
+  u64 room[2];        // rows of each buffer
+  u32* counts;        // three sets of COUNT_WORDS
+  u32 count_words;
+  u32 resume, phase0; // continue a stopped sweep from BinState
+  u32* born;          // per op: rows created
+  u64* anti;          // per op: rows anticommuting
+  u64* hist;          // noise ops: live count after
+  u64* stamps;        // device clock at the end of a window (its last op) / a solo op
+  SweepState* st;
+  BinState* bs;
+  u32 hold_block, hold_us;
+};
+
+template <int W, int ALG>
+int bins_grid();
+// Solo run of ops [op_begin, op_end) by one block, then the windows from
+// where it stopped (st->end_op) on the whole grid.
+template <int W, int ALG>
+cudaError_t launch_solo(const BinArgs& a, cudaStream_t s);
+template <int W, int ALG>
+cudaError_t launch_bins(const BinArgs& a, int grid, cudaStream_t s);
 
 enum : u32 { LOG_HELD = 0, LOG_L1 = 1, LOG_MAX = 2, LOG_EMITTED = 3, LOG_HITS = 4, LOG_WORDS = 5 };
 
