@@ -35,8 +35,14 @@
 // halves by further bits of the group hash, as often as it takes; nothing of
 // a bin is written before all of it has fitted.
 //
-// Small live sets run in one block with no grid barrier at all (solo_body):
-// all rows in shared memory, every op a step between two block barriers.
+// Who takes a bin follows the rows per bin: while a bin of every warp of the
+// grid holds the live set, each warp runs bins of its own, with no block
+// barrier anywhere in a window (and hands a bin that outgrows it to its
+// block); larger live sets go by blocks.  Small live sets run in one warp,
+// then one block, with no grid barrier at all (solo_run).  Windows whose
+// rotations all commute keep the set of rotations a term anticommutes with
+// fixed, so a bin of a few rows runs only the rotations one of them
+// anticommutes with.
 //
 // What bounds it: the dependent shared-memory round trips of a rotation's
 // step (about 1 us on small bins; 2-3 us where a block's 1,500-3,000 rows
@@ -52,6 +58,7 @@ constexpr u32 TAB_EMPTY = 0xffffffffu;
 constexpr u32 IDX_BITS = 13;  // row index bits of a shared-memory table slot, the rest is fingerprint
 constexpr u32 IDX_MASK = (1u << IDX_BITS) - 1u;
 
+// Rows of one unit -- a block (T = its threads) or a warp (T = 32).
 template <int W, int T_, int R_, int SLOTS_>
 struct BinSmem {
   static constexpr int T = T_, R = R_, SLOTS = SLOTS_;
@@ -59,20 +66,27 @@ struct BinSmem {
   double coef[R];
   u64 key[W][R];  // by word: lanes of consecutive rows read consecutive addresses
   u32 h[R];
-  u32 tab[SLOTS];
-  GateDesc<W> gate[4];  // ring: the running rotation and the next two
-  u64 pm[W];  // pivot bits of the next window's grouping
-  u32 hv[64 * W];  // per pivot bit: hash of its basis vector
-  u32 born[WIN_MAX], anti[WIN_MAX];    // this bin, per rotation
-  u32 born_all[WIN_MAX], anti_all[WIN_MAX];  // this block's bins of the window
-  OpDesc op[4];  // ring (solo)
-  unsigned short list[R];  // the running rotation's anticommuting rows
-  u32 n_list[2];           // their number; the other one is zero for the next rotation
-  unsigned char gate_of[64 * W];  // per pivot bit: the window's rotation it belongs to (disjoint windows)
-  u32 n, kept, tick;
-  u32 x[8];  // words read after a grid barrier
-  u64 y[4];
+  __align__(16) u32 tab[SLOTS];
+  __align__(16) GateDesc<W> gate[4];  // ring: the running rotation and the next two
+  u32 born[WIN_MAX];             // this bin, per rotation: rows created
+  unsigned short anti[WIN_MAX];  // ... rows anticommuting
+  unsigned short list[R];        // the running rotation's anticommuting rows
+  u32 n_list[2];                 // their number; the other one is zero for the next rotation
+  u32 act[WIN_MAX / 32];         // rotations to run (commuting windows, few rows)
+  __align__(8) WinDesc win[4];   // ring (solo): the running window and the next two
+  u32 n;
 };
+
+template <class S>
+__device__ __forceinline__ void unit_sync() {
+  if constexpr (S::T == 32) __syncwarp();
+  else __syncthreads();
+}
+template <class S>
+__device__ __forceinline__ int unit_tid() {
+  if constexpr (S::T == 32) return threadIdx.x & 31;
+  else return threadIdx.x;
+}
 
 // ------------------------------------------------------------ linear hash
 __device__ __forceinline__ u32 rotl32(u32 v, int r) { return r ? (v << r) | (v >> (32 - r)) : v; }
@@ -111,9 +125,9 @@ struct BinRules {
 // over the row; 0xffffffff (row 8191) cannot occur since rows stop below it.
 template <class S>
 __device__ __forceinline__ u32 tab_start(u32 h) {
-  constexpr int SHIFT = 33 - (S::SLOTS == 4096 ? 12 : (S::SLOTS == 8192 ? 13 : 14));
-  static_assert(S::SLOTS / 2 == 1 << (32 - SHIFT), "table size");
-  return (h * 0xC2B2AE35u) >> SHIFT;
+  constexpr u32 PAIRS = S::SLOTS / 2;
+  static_assert((PAIRS & (PAIRS - 1)) == 0, "table size");
+  return (h * 0xC2B2AE35u) / (u32)(0x100000000ull / PAIRS);
 }
 template <class S>
 __device__ __forceinline__ void tab_insert(S& s, u32 h, u32 row, u32 pair) {
@@ -138,7 +152,8 @@ __device__ __forceinline__ double flip(double v, bool neg) {  // v * -1.0 or v *
 // coefficients; children are appended from row n on (born counts them) and
 // inserted into the table, where no lookup of this rotation can match them
 // (their row is >= n).  Rows past the capacity are counted but not stored;
-// the caller sees n grow past R.  Block-wide; the caller's barrier ends it.
+// the caller sees n grow past R.  Run by the whole unit; the caller's barrier
+// ends it.
 //
 // Every row in a run without a TermBudget floor is within the weight cut (the
 // admission, each branch and each reclaim keep to it), so in a pair only the
@@ -146,10 +161,10 @@ __device__ __forceinline__ double flip(double v, bool neg) {  // v * -1.0 or v *
 // child alone.
 template <int W, int ALG, class S>
 __device__ __forceinline__ void rotate_rows(S& s, const GateDesc<W>& d, const BinRules& R, u32 n, u32 flip_flop,
-                                            u32* born, u32* anti) {
+                                            u32* born, unsigned short* anti) {
   using Ops = typename Alg<ALG>::T;
   constexpr int T = S::T, U = 4;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = unit_tid<S>(), lane = tid & 31, warp = tid >> 5;
   if ((u32)warp * 32u < n) {
     u32 bits = 0;
     for (u32 i = 0; i * T < n; i += U) {
@@ -184,11 +199,11 @@ __device__ __forceinline__ void rotate_rows(S& s, const GateDesc<W>& d, const Bi
       for (; bits; bits &= bits - 1) s.list[at++] = (unsigned short)((__ffs(bits) - 1) * T + tid);
     }
   }
-  __syncthreads();
+  unit_sync<S>();
   const u32 total = s.n_list[flip_flop];
   if (tid == 0) {
     s.n_list[flip_flop ^ 1] = 0;
-    *anti = total;
+    *anti = (unsigned short)total;
   }
   if (fabs(d.sn) < 1e-9) {  // OP_PHASE
     for (u32 i = tid; i < total; i += T) s.coef[s.list[i]] = __dmul_rn(s.coef[s.list[i]], d.cs);
@@ -263,9 +278,9 @@ __device__ __forceinline__ void rotate_rows(S& s, const GateDesc<W>& d, const Bi
   }
 }
 
-// Descriptors on their way into the ring (cp.async), by the block's last
-// warp, which has rows of its own only when the block is nearly full: its
-// waits overlap the other warps' work.
+// Descriptors on their way into the ring (cp.async), by the unit's last warp,
+// which has rows of its own only when the unit is nearly full: its waits
+// overlap the other warps' work.
 template <int W>
 __device__ __forceinline__ void fetch_gate(GateDesc<W>* dst, const GateDesc<W>* src) {
   constexpr u32 WORDS = sizeof(GateDesc<W>) / 8;
@@ -282,97 +297,177 @@ __device__ __forceinline__ void stamp_op(u64* stamps, u32 op) {
   stamps[op] = t;
 }
 
-// ------------------------------------------------------------ solo
-// One block runs ops from a.op_begin on while the rows fit its shared memory
-// (a gate may double them), then writes the rows out dense and leaves the op
-// it stopped before in st->end_op and the live count in st->n[0].
+template <class S>
+__device__ __forceinline__ void clear_table(S& s) {
+  for (int i = unit_tid<S>(); i < S::SLOTS / 4; i += S::T)
+    reinterpret_cast<uint4*>(s.tab)[i] = make_uint4(TAB_EMPTY, TAB_EMPTY, TAB_EMPTY, TAB_EMPTY);
+}
+
+// Which rotations [first, G) of a commuting window to run, for few rows: those
+// some row anticommutes with (the rows they create anticommute with the same
+// ones).  Between barriers of the caller.  A lane tests one rotation against
+// every row.
+constexpr u32 ACT_ROWS = 64;
 template <int W, int ALG, class S>
-__device__ __forceinline__ void solo_body(const BinArgs& a, S& s) {
+__device__ __forceinline__ void find_active(S& s, const GateDesc<W>* gates, u32 first, u32 G, u32 n) {
+  for (u32 g0 = first & ~31u; g0 < WIN_MAX; g0 += S::T) {
+    const u32 g = g0 + unit_tid<S>();
+    bool on = false;
+    if (g >= first && g < G) {
+      u64 am[W];
+#pragma unroll
+      for (int w = 0; w < W; ++w) am[w] = anti_word<W, ALG>(gates[g], w);
+      for (u32 r = 0; r < n && !on; ++r) {
+        u64 acc = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) acc ^= s.key[w][r] & am[w];
+        on = popc(acc) & 1;
+      }
+    }
+    const unsigned m = __ballot_sync(FULL, on);
+    if ((threadIdx.x & 31) == 0 && g < WIN_MAX) s.act[g >> 5] = m;
+  }
+}
+// The next rotation to run from g on (G: none).  `some`: by s.act, else all.
+template <class S>
+__device__ __forceinline__ u32 next_gate(const S& s, bool some, u32 g, u32 G) {
+  if (!some || g >= G) return g < G ? g : G;
+  u32 w = g >> 5, m = s.act[w] & (~0u << (g & 31u));
+  while (!m) {
+    if (++w * 32 >= G) return G;
+    m = s.act[w];
+  }
+  g = 32 * w + __ffs(m) - 1;
+  return g < G ? g : G;
+}
+
+// ------------------------------------------------------------ solo
+// One unit runs windows from (win, first) on while the rows fit it (a rotation
+// may double them), from and to the dense rows.  Returns with win / first at
+// the rotation it stopped before (win == n_windows at the end) and n the live
+// count.  Its rows must number at most R / 2 at entry.
+template <int W, int ALG, class S>
+__device__ __noinline__ void solo_run(const BinArgs& a, S& s, u32& win, u32& first, u32& n_io) {
   using Ops = typename Alg<ALG>::T;
   constexpr int T = S::T;
-  const int tid = threadIdx.x, lane = tid & 31;
-  SweepState* st = a.st;
+  constexpr u32 NONE = 0xffffffffu;
+  const int tid = unit_tid<S>(), lane = tid & 31;
+  const bool fetcher = tid >= T - 32;
   const GateDesc<W>* gates = reinterpret_cast<const GateDesc<W>*>(a.gates);
-  u32 op = a.op_begin;
-  const u64 n_in = a.n0;
-  if (n_in > (u64)S::R / 2) {
-    if (tid == 0) {
-      st->n[0] = n_in;
-      st->end_op = op;
-    }
-    return;
-  }
-  u32 n = (u32)n_in;
-  auto clear_table = [&] {
-    for (int i = tid; i < S::SLOTS / 4; i += T)
-      reinterpret_cast<uint4*>(s.tab)[i] = make_uint4(TAB_EMPTY, TAB_EMPTY, TAB_EMPTY, TAB_EMPTY);
+  u32 n = n_io;
+  auto fetch_window = [&](u32 x) {  // by the fetcher: window x into its place of the ring
+    constexpr u32 WORDS = sizeof(WinDesc) / 8;
+    if (x < a.n_windows && lane < (int)WORDS)
+      cp_async8(reinterpret_cast<u64*>(&s.win[x & 3]) + lane, reinterpret_cast<const u64*>(a.windows + x) + lane);
   };
-  clear_table();
-  if (tid < 4) s.born[tid] = s.anti[tid] = 0;
+  clear_table(s);
+  if (tid < 4) s.born[tid] = 0;
   if (tid < 2) s.n_list[tid] = 0;
-  __syncthreads();
+  if (fetcher) {
+    fetch_window(win);
+    fetch_window(win + 1);
+    cp_async_wait();
+  }
+  unit_sync<S>();
   for (u32 r = tid; r < n; r += T) {
     u64 k[W];
     load_key<W>(a.keys, r, k);
     const u32 h = lin_hash<W>(k, a.lin);
 #pragma unroll
     for (int w = 0; w < W; ++w) s.key[w][r] = k[w];
-    s.coef[r] = a.coeffs[r];
+    s.coef[r] = __ldcg(a.coeffs + r);
     s.h[r] = h;
     tab_insert(s, h, r, tab_start<S>(h));
   }
   BinRules R;
   R.n_units = a.n_units;
   R.minc = a.min_coeff;
-  u32 step = 0;  // rotations run: their counters are born / anti [step & 3]
-  u32 last = 0xffffffffu;   // op whose counters are in born[(step - 1) & 3], not yet taken
-  const bool fetcher = tid >= T - 32;
+  R.wcut = a.max_weight;
+  R.ccut = a.has_min_coeff != 0;
+  u32 step = 0;          // rotations run: counters born / anti [step & 3], descriptor gate[step & 3]
+  u32 last = NONE;       // op whose counters are in [(step - 1) & 3], not yet taken
+  u32 pa = NONE, pb = NONE;  // descriptors on their way for this step and the next
   // The live count after the last rotation; thread 0 records its counters.
   auto take = [&] {
-    if (last == 0xffffffffu) return;
+    if (last == NONE) return;
     const u32 b = s.born[(step - 1) & 3];
     n += b;
     if (tid == 0) {
       a.born[last] = b;
       a.anti[last] = s.anti[(step - 1) & 3];
     }
-    last = 0xffffffffu;
+    last = NONE;
   };
-  // Rings: ops op, op + 1 (and, while op runs, op + 2); the next rotation's
-  // descriptor (gate index gi), the one after, and gi + 2 while gi runs.
-  u32 gi = a.first_gate;
-  if (fetcher) {
-    if (lane < 2 && op + lane < a.op_end) cp_async8(&s.op[(op + lane) & 3], a.ops + op + lane);
-    for (u32 g = gi; g < gi + 2 && g < a.n_gdesc; ++g) fetch_gate<W>(&s.gate[g & 3], gates + g);
-    cp_async_wait();
-  }
-  while (op < a.op_end) {
-    if (fetcher) cp_async_wait_1();
-    __syncthreads();  // the step before is done; this op's descriptors are here
-    take();
-    const OpDesc od = s.op[op & 3];
-    const bool rot = od.kind == OP_GATE || od.kind == OP_PHASE;
-    if (od.kind == OP_GATE && 2 * n > (u32)S::R) break;
+  bool stop = false;
+  while (win < a.n_windows) {
+    // Fetched while the window before the last began; every window waits for
+    // all but its latest fetch and then meets a barrier, so it is here.
+    bool met = false;
+    const WinDesc& w = s.win[win & 3];
     if (fetcher) {
-      if (lane == 0 && op + 2 < a.op_end) cp_async8(&s.op[(op + 2) & 3], a.ops + op + 2);
-      if (rot && gi + 2 < a.n_gdesc) fetch_gate<W>(&s.gate[(gi + 2) & 3], gates + gi + 2);
+      fetch_window(win + 2);
       cp_async_commit();
     }
-    if (rot) {
-      if (tid == 0) s.born[(step + 2) & 3] = 0;
-      R.wcut = a.max_weight;
-      R.ccut = a.has_min_coeff != 0;
-      rotate_rows<W, ALG>(s, s.gate[gi & 3], R, n, step & 1, &s.born[step & 3], &s.anti[step & 3]);
-      last = op;
-      ++step;
-      ++gi;
-    } else {
-      const double* factors = a.tables + (u64)od.idx * a.table_len;
+    const u32 G = w.n_gates;
+    if (first < G) {
+      bool some = false;
+      if (w.commute && G - first > 4) {
+        unit_sync<S>();
+        take();
+        some = n <= ACT_ROWS;
+        if (some) {
+          find_active<W, ALG>(s, gates + w.gate, first, G, n);
+          unit_sync<S>();
+        }
+      }
+      u32 g = next_gate(s, some, first, G);
+      while (g < G) {
+        const u32 g1 = next_gate(s, some, g + 1, G), g2 = next_gate(s, some, g1 + 1, G);
+        const u32 id = w.gate + g, id1 = w.gate + (g1 < G ? g1 : G), id2 = g1 < G ? w.gate + (g2 < G ? g2 : G) : id1 + 1;
+        if (pa != id) {  // not the one that was expected: now, with the next
+          if (fetcher) {
+            cp_async_wait();
+            fetch_gate<W>(&s.gate[step & 3], gates + id);
+            if (id1 < a.n_gdesc) fetch_gate<W>(&s.gate[(step + 1) & 3], gates + id1);
+            cp_async_wait();
+          }
+          pb = id1;
+        } else if (fetcher) {
+          cp_async_wait_1();
+        }
+        unit_sync<S>();  // the step before is done; this rotation's descriptor is here
+        met = true;
+        take();
+        if (2 * n > (u32)S::R) {
+          stop = true;
+          break;
+        }
+        if (fetcher) {
+          if (id2 < a.n_gdesc) fetch_gate<W>(&s.gate[(step + 2) & 3], gates + id2);
+          cp_async_commit();
+        }
+        pa = pb;
+        pb = id2;
+        if (tid == 0) s.born[(step + 2) & 3] = 0;
+        rotate_rows<W, ALG>(s, s.gate[step & 3], R, n, step & 1, &s.born[step & 3], &s.anti[step & 3]);
+        last = w.op + g;
+        ++step;
+        g = g1;
+      }
+      first = g;
+      if (stop) break;
+    }
+    if (w.noise) {
+      if (fetcher) cp_async_wait_1();
+      unit_sync<S>();
+      met = true;
+      take();
+      const double* factors = a.tables + (u64)w.table * a.table_len;
       const u32 lastw = a.table_len - 1;
-      const bool reclaim = od.kind == OP_NOISE_COMPACT;
+      const bool reclaim = w.noise == 2;
       if (reclaim) {
         if (tid == 0) s.n = 0;
-        clear_table();
+        clear_table(s);
       }
       // T rows a round: all of a round are in registers before any is written
       // back, and the survivors of the first i rounds never reach row i T.
@@ -384,7 +479,7 @@ __device__ __forceinline__ void solo_body(const BinArgs& a, S& s) {
         bool kp = false;
         if (r < n) {
 #pragma unroll
-          for (int w = 0; w < W; ++w) k[w] = s.key[w][r];
+          for (int x = 0; x < W; ++x) k[x] = s.key[x][r];
           h = s.h[r];
           const u32 wt = Ops::template weight<W>(k, a.n_units);
           c = __dmul_rn(s.coef[r], __ldg(factors + (wt < lastw ? wt : lastw)));
@@ -395,7 +490,7 @@ __device__ __forceinline__ void solo_body(const BinArgs& a, S& s) {
                  (!a.has_min_coeff || fabs(c) >= a.min_coeff);
         }
         if (!reclaim) continue;
-        __syncthreads();
+        unit_sync<S>();
         const unsigned m = __ballot_sync(FULL, kp);
         if (!m) continue;
         u32 at = 0;
@@ -403,58 +498,118 @@ __device__ __forceinline__ void solo_body(const BinArgs& a, S& s) {
         at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
         if (!kp) continue;
 #pragma unroll
-        for (int w = 0; w < W; ++w) s.key[w][at] = k[w];
+        for (int x = 0; x < W; ++x) s.key[x][at] = k[x];
         s.coef[at] = c;
         s.h[at] = h;
         tab_insert(s, h, at, tab_start<S>(h));
       }
       if (reclaim) {
-        __syncthreads();
+        unit_sync<S>();
         n = s.n;
       }
-      if (tid == 0) a.hist[op] = n;
+      if (tid == 0) a.hist[w.op + G] = n;
     }
-    if (tid == T - 1 && (op + 1 == a.op_end || (s.op[(op + 1) & 3].kind == OP_NOISE_COMPACT) !=
-                                                   (od.kind == OP_NOISE_COMPACT)))
-      stamp_op(a.stamps, op);
-    ++op;
+    // (reading the clock takes about as long as a rotation)
+    if (tid == T - 1 && ((win & 7u) == 7u || win + 1 == a.n_windows)) stamp_op(a.stamps, w.op_end - 1);
+    if (!met) {
+      if (fetcher) cp_async_wait_1();
+      unit_sync<S>();
+    }
+    ++win;
+    first = 0;
   }
-  __syncthreads();
+  unit_sync<S>();
   take();
   if (fetcher) cp_async_wait();
   for (u32 r = tid; r < n; r += T) {
     u64 k[W];
 #pragma unroll
-    for (int w = 0; w < W; ++w) k[w] = s.key[w][r];
+    for (int x = 0; x < W; ++x) k[x] = s.key[x][r];
     store_key<W>(a.keys, r, k);
     a.coeffs[r] = s.coef[r];
   }
-  if (tid == 0) {
+  n_io = n;
+}
+
+// The window op `op` lies in (windows cover every op in order).
+__device__ __forceinline__ u32 window_of(const BinArgs& a, u32 op) {
+  u32 lo = 0, hi = a.n_windows;
+  while (lo < hi) {
+    const u32 mid = (lo + hi) / 2;
+    if (a.windows[mid].op_end <= op) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// A block alone: its first warp while the rows fit it, then all of it; leaves
+// the op it stopped before in st->end_op and the live count in st->n[0].
+template <int W, int ALG, class SW, class SB>
+__device__ __forceinline__ void solo_body(const BinArgs& a, SW& sw, SB& sb) {
+  SweepState* st = a.st;
+  u32 win = window_of(a, a.op_begin), first = 0, n = 0;
+  if (win < a.n_windows && a.op_begin > a.windows[win].op) first = a.op_begin - a.windows[win].op;
+  const u64 n0 = a.n0;
+  if (n0 > (u64)SB::R / 2 || win >= a.n_windows) {
+    if (threadIdx.x == 0) {
+      st->n[0] = n0;
+      st->end_op = win < a.n_windows ? a.op_begin : a.op_end;
+    }
+    return;
+  }
+  n = (u32)n0;
+  if (n <= (u32)SW::R / 2) {
+    __shared__ u32 hand[3];
+    if (threadIdx.x < 32) {
+      solo_run<W, ALG>(a, sw, win, first, n);
+      if (threadIdx.x == 0) {
+        hand[0] = win;
+        hand[1] = first;
+        hand[2] = n;
+      }
+    }
+    __syncthreads();
+    win = hand[0];
+    first = hand[1];
+    n = hand[2];
+  }
+  if (win < a.n_windows) solo_run<W, ALG>(a, sb, win, first, n);
+  if (threadIdx.x == 0) {
     st->n[0] = n;
-    st->end_op = op;
+    st->end_op = win < a.n_windows ? a.windows[win].op + first : a.op_end;
   }
 }
 
 // ------------------------------------------------------------ binned windows
 // The bins the rows are dealt into: bin b holds rows [b * cap, b * cap +
 // count[b]) of its buffer, and rows past a full bin go to the buffer's spill
-// area, tagged with their bin.  to == 0xffffffff: dense, no bins (the end of
-// the sweep).
+// area, tagged with their bin.
 constexpr u64 SPILL_SHARE = 16;  // of a buffer; more spills than that and the host grows it
 struct Layout {
   u32 bins, stride;  // counters are `stride` words apart (few bins: a sector or line each)
   u32 cap;
 };
 
-// Bins for about n rows, m of them each, in a buffer of `room` rows: never
-// fewer than the blocks, all the room there is (less an eighth for spills).
-__device__ __forceinline__ Layout choose_layout(u64 n, u32 m, u32 blocks, u64 room) {
+// Bins for about n rows that a window lets grow by a factor `grow`, grown bins
+// `fill` full.  While a bin of every warp holds at most WARP_ROWS rows when
+// grown, that many (a warp alone runs 32 branching rows at a time, a block
+// 256: bins that grew to 62 rows a warp ran a window of 50 rotations in 79 us
+// (kicked Ising 10x10) against 72 us by blocks, bins of 22 one of 40 in 43
+// against 51 us; where one family fills a bin, as in a TFIM chain's RX layer,
+// the line is lower); else bins of blocks, one each or, up to four, a whole
+// number each (340 bins on 296 blocks cost two rounds).  All the room there
+// is, less the spill area.
+constexpr float WARP_ROWS = 12.0f;
+__device__ __forceinline__ Layout choose_layout(float n, float grow, float fill, u32 blocks, u32 warps, u32 rows,
+                                                u64 room) {
   Layout l;
-  u64 b = (n + m - 1) / m;
-  if (b < blocks) b = blocks;
+  u64 b = (u64)(n * grow / (fill * (float)rows)) + 1;
+  if (n * grow <= WARP_ROWS * (float)(blocks * warps)) b = (u64)blocks * warps;
+  else if (b < 4ull * blocks) b = (b + blocks - 1) / blocks * blocks;
+  else if (b == (u64)blocks * warps) ++b;  // that number means bins of warps
   if (b > BIN_MAX) b = BIN_MAX;
   l.bins = (u32)b;
-  l.stride = b <= 2048 ? 32u : (b <= 16384 ? 4u : 1u);
+  l.stride = b <= 4096 ? 32u : (b <= 16384 ? 8u : 1u);
   const u64 c = (room - room / SPILL_SHARE) / b;
   l.cap = c > 0x7fffffffull ? 0x7fffffffu : (u32)c;
   return l;
@@ -466,7 +621,7 @@ __device__ __forceinline__ u32 split_bits(u32 g) { return (g ^ (g >> 15)) * 0x85
 
 // Group hash from the basis list itself (the slow way: splits only).
 template <int W, int ALG>
-__device__ u32 group_hash_list(const u64* k, u32 h, const BinArgs& a, const WinDesc& w) {
+__device__ __noinline__ u32 group_hash_list(const u64* k, u32 h, const BinArgs& a, const WinDesc& w) {
   const GateDesc<W>* gates = reinterpret_cast<const GateDesc<W>*>(a.gates);
   for (u32 i = 0; i < w.n_basis; ++i) {
     const BasisDesc b = a.basis[w.basis + i];
@@ -482,58 +637,82 @@ __device__ u32 group_hash_list(const u64* k, u32 h, const BinArgs& a, const WinD
   return h;
 }
 
-template <int W, int ALG, class S>
-__device__ __forceinline__ u32 group_hash(const S& s, const u64* k, u32 h, const GateDesc<W>* gates, const WinDesc& w) {
-#pragma unroll
-  for (int x = 0; x < W; ++x)
-    for (u64 m = k[x] & s.pm[x]; m; m &= m - 1) {
-      const int bit = 64 * x + __ffsll((long long)m) - 1;
-      if (w.disjoint) {
-        const GateDesc<W>& d = gates[w.gate + s.gate_of[bit]];
-        u64 acc = 0;
-#pragma unroll
-        for (int y = 0; y < W; ++y) acc ^= k[y] & __ldg(&d.g.fold[y]);
-        if (!(popc(acc) & 1)) continue;
-      }
-      h ^= s.hv[bit];
-    }
-  return h;
-}
-
-// Loads the grouping of window w into shared memory.
-template <int W, class S>
-__device__ __forceinline__ void load_grouping(S& s, const BinArgs& a, const WinDesc& w) {
-  if (threadIdx.x < W) s.pm[threadIdx.x] = 0;
-  __syncthreads();
-  for (u32 i = threadIdx.x; i < w.n_basis; i += S::T) {
-    const BasisDesc b = a.basis[w.basis + i];
-    s.hv[b.bit] = b.hash;
-    s.gate_of[b.bit] = (unsigned char)b.gate;
-    atomicOr(&s.pm[b.bit >> 6], 1ull << (b.bit & 63));
-  }
-  __syncthreads();
-}
-
-// Where finished rows go: into the bins of window `w` (layout `l`, buffer
-// `buf`, counters `cnt`), or dense.
-template <int W>
+// Where finished rows go: into the bins of the next window (layout `l`,
+// counters `cnt`), or dense.
 struct Dest {
-  bool dense;
-  Layout l;
   u64* keys;
   double* coeffs;
   u32* h;
   u32* cnt;
   u32* spill_bin;
-  u64 room;        // rows of the buffer (bins, then spills)
   u32* n_spill;    // spilled rows
-  u64* n_dense;    // dense: rows written
+  u64* n_dense;    // dense (no bins): rows written
   u32* fail;       // set when the buffer is full
+  u64 room;        // rows of the buffer (bins, then spills)
+  Layout l;
+  u32 dense;
 };
 
-template <int W, int ALG, class S>
-__device__ __forceinline__ void put_row(const S& s, const Dest<W>& d, const u64* k, double c, u32 h, bool act,
-                                        const GateDesc<W>* gates, const WinDesc& w) {
+// What every unit of a block shares in a window.
+template <int W>
+struct WinSmem {
+  u64 pm[W];       // pivot bits of the next window's grouping
+  u32 hv[64 * W];  // per pivot bit: hash of its basis vector
+  unsigned char gate_of[64 * W];  // per pivot bit: the next window's rotation it belongs to (disjoint windows)
+  u32 born_all[WIN_MAX], anti_all[WIN_MAX];  // this block's bins, per rotation
+  WinDesc w, wn;
+  Dest d;
+  // the rows of this window's bins
+  const u64* bk;
+  const double* bc;
+  const u32* bh;
+  const u32* bsp;
+  const u32* cnt;
+  u64 y[2];       // words read after the grid barrier
+  u32 x[2];
+  Layout lay, prev;
+  u32 spilled, first;
+  float grow;     // expected growth of this window's bins, at least 1
+  u32 kept, tick, n_defer;
+  u32 defer[32];  // bins the block's warps could not hold
+};
+
+template <int W, int ALG>
+__device__ __forceinline__ u32 group_hash(const WinSmem<W>& v, const u64* k, u32 h, const GateDesc<W>* gates) {
+#pragma unroll
+  for (int x = 0; x < W; ++x)
+    for (u64 m = k[x] & v.pm[x]; m; m &= m - 1) {
+      const int bit = 64 * x + __ffsll((long long)m) - 1;
+      if (v.wn.disjoint) {
+        const GateDesc<W>& d = gates[v.wn.gate + v.gate_of[bit]];
+        u64 acc = 0;
+#pragma unroll
+        for (int y = 0; y < W; ++y) acc ^= k[y] & __ldg(&d.g.fold[y]);
+        if (!(popc(acc) & 1)) continue;
+      }
+      h ^= v.hv[bit];
+    }
+  return h;
+}
+
+// Loads the grouping of window v.wn (after v.wn is visible to the block).
+template <int W>
+__device__ __forceinline__ void load_grouping(WinSmem<W>& v, const BinArgs& a) {
+  if (threadIdx.x < W) v.pm[threadIdx.x] = 0;
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < v.wn.n_basis; i += blockDim.x) {
+    const BasisDesc b = a.basis[v.wn.basis + i];
+    v.hv[b.bit] = b.hash;
+    v.gate_of[b.bit] = (unsigned char)b.gate;
+    atomicOr(&v.pm[b.bit >> 6], 1ull << (b.bit & 63));
+  }
+  __syncthreads();
+}
+
+template <int W, int ALG>
+__device__ __forceinline__ void put_row(const WinSmem<W>& v, const u64* k, double c, u32 h, bool act,
+                                        const GateDesc<W>* gates) {
+  const Dest& d = v.d;
   u64 at;
   if (d.dense) {
     const unsigned m = __ballot_sync(FULL, act);
@@ -549,14 +728,13 @@ __device__ __forceinline__ void put_row(const S& s, const Dest<W>& d, const u64*
     }
   } else {
     if (!act) return;
-    const u32 bin = bin_of(group_hash<W, ALG>(s, k, h, gates, w), d.l.bins);
+    const u32 bin = bin_of(group_hash<W, ALG>(v, k, h, gates), d.l.bins);
     const u32 pos = atomicAdd(d.cnt + (u64)bin * d.l.stride, 1u);
     if (pos < d.l.cap) {
       at = (u64)bin * d.l.cap + pos;
     } else {
-      const u64 first = (u64)d.l.bins * d.l.cap;
       const u32 sp = atomicAdd(d.n_spill, 1u);
-      at = first + sp;
+      at = (u64)d.l.bins * d.l.cap + sp;
       if (at >= d.room) {
         *d.fail = 1;
         return;
@@ -569,45 +747,264 @@ __device__ __forceinline__ void put_row(const S& s, const Dest<W>& d, const u64*
   d.coeffs[at] = c;
 }
 
-template <int W, int ALG, class S>
-__device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, S& s) {
+// A finished row (1 if it is kept): the reclaim after the window, then its
+// next bin.  Called by whole warps.
+template <int W, int ALG>
+__device__ __forceinline__ u32 finish_row_body(const WinSmem<W>& v, const BinArgs& a, const u64 (&k)[W], double c,
+                                               u32 h, bool act) {
   using Ops = typename Alg<ALG>::T;
+  if (act && v.w.noise) {
+    const u32 lastw = a.table_len - 1;
+    const u32 wt = Ops::template weight<W>(k, a.n_units);
+    c = __dmul_rn(c, __ldg(a.tables + (u64)v.w.table * a.table_len + (wt < lastw ? wt : lastw)));
+    if (v.w.noise == 2)
+      act = (a.max_weight == NO_WEIGHT_CUT || wt <= a.max_weight) && (!a.has_min_coeff || fabs(c) >= a.min_coeff);
+  }
+  put_row<W, ALG>(v, k, c, h, act, reinterpret_cast<const GateDesc<W>*>(a.gates));
+  return act ? 1u : 0u;
+}
+template <int W, int ALG>
+__device__ __noinline__ u32 finish_row_call(const WinSmem<W>& v, const BinArgs& a, const u64 (&k)[W], double c, u32 h,
+                                            bool act) {
+  return finish_row_body<W, ALG>(v, a, k, c, h, act);
+}
+// Inlined at its four places it makes the 4- and 8-word kernels spill (kicked
+// Ising 12x15 4.6 -> 5.6 ms); a call costs the narrow ones (6x6 2.14 -> 2.24).
+template <int W, int ALG>
+__device__ __forceinline__ u32 finish_row(const WinSmem<W>& v, const BinArgs& a, const u64 (&k)[W], double c, u32 h,
+                                          bool act) {
+  if constexpr (W <= 2) return finish_row_body<W, ALG>(v, a, k, c, h, act);
+  else return finish_row_call<W, ALG>(v, a, k, c, h, act);
+}
+
+// One bin by one unit: its rows into shared memory, the window's rotations,
+// and every row on to its next place.  A block splits what does not fit; a
+// warp returns false instead, having written nothing.  depth0: how deep this
+// block's bins of the window have been split so far.
+template <int W, int ALG, class S>
+__device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u32 bin, u32& depth0, u32& kept) {
   constexpr int T = S::T;
-  const int tid = threadIdx.x, lane = tid & 31;
+  constexpr bool WARP = T == 32;
+  constexpr u32 NONE = 0xffffffffu;
+  const int tid = unit_tid<S>();
   const bool fetcher = tid >= T - 32;
+  const u32 n_all = __ldcg(v.cnt + (u64)bin * v.lay.stride);
+  if (!n_all) return true;
+  const u32 n_bin = n_all < v.lay.cap ? n_all : v.lay.cap;
+  const bool has_spill = n_all > v.lay.cap;
+  const u64 row0 = (u64)bin * v.lay.cap, spill0 = (u64)v.lay.bins * v.lay.cap;
+  const u32 G = v.w.n_gates, first = v.first, spilled = v.spilled;
+  if (first >= G) {  // no rotation: straight through
+    for (u32 r0 = 0; r0 < n_bin + (has_spill ? spilled : 0u); r0 += T) {
+      const u32 r = r0 + tid;
+      const bool in_bin = r < n_bin;
+      const u64 src = in_bin ? row0 + r : spill0 + (r - n_bin);
+      const bool act = in_bin || (has_spill && r < n_bin + spilled && __ldcg(v.bsp + (r - n_bin)) == bin);
+      u64 k[W];
+      double c = 0.0;
+      u32 h = 0;
+      if (act) {
+        load_key<W>(v.bk, src, k);
+        c = __ldcg(v.bc + src);
+        h = __ldcg(v.bh + src);
+      }
+      kept += finish_row<W, ALG>(v, a, k, c, h, act);
+    }
+    return true;
+  }
+  // A warp runs its bin whole or not at all (a part that did not fit after
+  // another was written would be run twice).
+  if (WARP && (has_spill || n_all > (u32)S::R / 2)) return false;
+  const GateDesc<W>* gates = reinterpret_cast<const GateDesc<W>*>(a.gates) + v.w.gate;
+  BinRules R;
+  R.n_units = a.n_units;
+  R.minc = a.min_coeff;
+  R.wcut = a.max_weight;
+  R.ccut = a.has_min_coeff != 0;
+  // Parts of the bin: `part` of 2^depth by split_bits, in order.
+  u32 depth = WARP ? 0 : depth0, part = 0;
+  // split at once what would outgrow the unit at the expected growth: failing
+  // late in a window of 80 rotations takes as long as running it
+  while (!WARP && depth < 24 && (float)(n_all >> depth) * v.grow > (float)S::R * 0.9f) ++depth;
+  const u32 base = depth;
+  for (;;) {
+    for (u32 i = tid; i < G; i += T) {
+      s.born[i] = 0;
+      s.anti[i] = 0;
+    }
+    clear_table(s);
+    if (tid == 0) s.n = s.n_list[0] = s.n_list[1] = 0;
+    unit_sync<S>();
+    u32 n = n_all;
+    if (depth == 0 && !has_spill) {
+      for (u32 r = tid; r < n_bin; r += T) {
+        u64 k[W];
+        load_key<W>(v.bk, row0 + r, k);
+        const double c = __ldcg(v.bc + row0 + r);
+        const u32 h = __ldcg(v.bh + row0 + r);
+#pragma unroll
+        for (int x = 0; x < W; ++x) s.key[x][r] = k[x];
+        s.coef[r] = c;
+        s.h[r] = h;
+        tab_insert(s, h, r, tab_start<S>(h));
+      }
+    } else {
+      auto take = [&](u64 src) {
+        u64 k[W];
+        load_key<W>(v.bk, src, k);
+        const u32 h = __ldcg(v.bh + src);
+        if (depth && (split_bits(group_hash_list<W, ALG>(k, h, a, v.w)) >> (32 - depth)) != part) return;
+        const u32 r = atomicAdd(&s.n, 1u);
+        if (r >= (u32)S::R) return;
+#pragma unroll
+        for (int x = 0; x < W; ++x) s.key[x][r] = k[x];
+        s.coef[r] = __ldcg(v.bc + src);
+        s.h[r] = h;
+        tab_insert(s, h, r, tab_start<S>(h));
+      };
+      for (u32 r = tid; r < n_bin; r += T) take(row0 + r);
+      if (has_spill)
+        for (u32 r = tid; r < spilled; r += T)
+          if (__ldcg(v.bsp + r) == bin) take(spill0 + r);
+      unit_sync<S>();
+      n = s.n;
+    }
+    bool fits = n <= (u32)S::R;
+    if (fits) {
+      const bool some = v.w.commute && n <= ACT_ROWS;
+      if (some) {
+        unit_sync<S>();
+        find_active<W, ALG>(s, gates, first, G, n);
+        unit_sync<S>();
+      }
+      u32 g = next_gate(s, some, first, G), before = NONE, step = 0;
+      u32 g1 = next_gate(s, some, g + 1, G);
+      if (fetcher && g < G) {
+        fetch_gate<W>(&s.gate[0], gates + g);
+        if (g1 < G) fetch_gate<W>(&s.gate[1], gates + g1);
+        cp_async_wait();
+      }
+      for (; g < G; ++step) {
+        if (fetcher) cp_async_wait_1();
+        unit_sync<S>();
+        if (before != NONE) {
+          n += s.born[before];
+          if (n > (u32)S::R) {
+            fits = false;
+            break;
+          }
+        }
+        const u32 g2 = next_gate(s, some, g1 + 1, G);
+        if (fetcher) {
+          if (g2 < G) fetch_gate<W>(&s.gate[(step + 2) & 3], gates + g2);
+          cp_async_commit();
+        }
+        rotate_rows<W, ALG>(s, s.gate[step & 3], R, n, step & 1, &s.born[g], &s.anti[g]);
+        before = g;
+        g = g1;
+        g1 = g2;
+      }
+      if (fetcher) cp_async_wait();
+      unit_sync<S>();
+      if (fits && before != NONE) {
+        n += s.born[before];
+        fits = n <= (u32)S::R;
+      }
+    }
+    if (!fits) {
+      if (WARP) return false;
+      ++depth;  // run the part again in halves
+      part <<= 1;
+      if (depth0 < depth && depth0 < 8) depth0 = depth;
+      if (depth > 24) {
+        if (tid == 0) atomicOr(&a.st->error, ERR_CAPACITY);
+        return true;
+      }
+      unit_sync<S>();
+      continue;
+    }
+    for (u32 i = tid; i < G; i += T) {
+      if (s.born[i]) atomicAdd(&v.born_all[i], s.born[i]);
+      if (s.anti[i]) atomicAdd(&v.anti_all[i], (u32)s.anti[i]);
+    }
+    for (u32 r0 = 0; r0 < n; r0 += T) {
+      const u32 r = r0 + tid;
+      u64 k[W];
+      double c = 0.0;
+      u32 h = 0;
+      if (r < n) {
+#pragma unroll
+        for (int x = 0; x < W; ++x) k[x] = s.key[x][r];
+        c = s.coef[r];
+        h = s.h[r];
+      }
+      kept += finish_row<W, ALG>(v, a, k, c, h, r < n);
+    }
+    unit_sync<S>();
+    while (depth && (part & 1u)) {
+      part >>= 1;
+      --depth;
+    }
+    if (!depth) return true;
+    ++part;
+    while (depth < base) {
+      ++depth;
+      part <<= 1;
+    }
+  }
+}
+
+// The windows from where the solo run (or a stopped sweep) left off, by the
+// blocks of grp.  SB: a block's rows, SW: a warp's; both lie over one another
+// in `rows`.
+template <int W, int ALG, class SB, class SW>
+__device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSmem<W>& v, SB& sb, SW* sw) {
+  constexpr int T = SB::T, WARPS = T / 32;
+  const int tid = threadIdx.x, lane = tid & 31;
   SweepState* st = a.st;
   BinState* bs = a.bs;
   const GateDesc<W>* gates = reinterpret_cast<const GateDesc<W>*>(a.gates);
   u32 gen = *(volatile u32*)&st->bar_gen;
   if (a.hold_us && grp.bid == a.hold_block && tid == 0) hold(a.hold_us);
 
-  // Position: the window, the first rotation of it still to run, the buffer
-  // and counter set holding the rows (ph), or the dense rows at entry.
+  // Position: the window, the first rotation of it still to run, and the
+  // number of buffer fills so far: fill ph lies in buffer ph & 1, its counters
+  // in set ph % 3.
   const bool resumed = a.resume != 0;
   const u32 op_start = resumed ? bs->op : *(volatile u32*)&st->end_op;
   u64 N = resumed ? bs->rows : ld_volatile(&st->n[0]);
-  u32 win = a.n_windows, first = 0;
-  {  // the window op_start lies in (windows cover every op in order)
-    u32 lo = 0, hi = a.n_windows;
-    while (lo < hi) {
-      const u32 mid = (lo + hi) / 2;
-      if (a.windows[mid].op_end <= op_start) lo = mid + 1;
-      else hi = mid;
-    }
-    win = lo;
-  }
+  u32 win = window_of(a, op_start);
   if (win >= a.n_windows) return;  // nothing left (the dense rows are the result)
-  {
-    const WinDesc& w0 = a.windows[win];
-    first = op_start > w0.op ? op_start - w0.op : 0;
-  }
+  u32 first = op_start > a.windows[win].op ? op_start - a.windows[win].op : 0;
   u32 ph = resumed ? bs->phase : 0;
   Layout lay = resumed ? Layout{bs->bins, bs->stride, bs->cap} : Layout{0, 0, 0};
-  float rho = resumed ? bs->rho : 1.5f;  // growth of the live count inside recent windows
 
+  // The layout for window x, entered by about n rows.  How they will grow: as
+  // in an earlier window of the same rotations (host: WinDesc::like), if that
+  // was entered by about as many rows, else as in the windows just before.
+  // Bins 85% full where that is known and steady.  Less where the growth is
+  // steep, for then it is uneven (kicked Ising 6x6, x18 in an RX layer: 381
+  // -> 214 us at 45%), or not known, the more so the longer the window: a bin
+  // that does not fit after all is run again in halves.
+  float rho = resumed ? bs->rho : 1.5f;
+  auto alike = [&](float n, u32 x) -> const float* {
+    const u32 like = a.windows[x].like;
+    if (like == 0xffffffffu) return nullptr;
+    const float* h = a.growth + 3 * like;
+    const float was = __ldcg(h + 2);
+    return was > 0.0f && n < 8.0f * was && was < 8.0f * n ? h : nullptr;
+  };
+  float next_grow = resumed ? bs->grow : 1.0f;  // expected growth of the window dealt to last
+  auto layout_for = [&](float n, u32 x, u64 room) {
+    const float* h = alike(n, x);
+    const float g = h ? fmaxf(__ldcg(h), 1.0f) : fminf(fmaxf(1.15f * rho, 1.5f), 3.0f);
+    next_grow = 1.0f + 0.5f * (g - 1.0f);  // bins differ: followed half way
+    const float fill = h ? (g < 3.0f ? 0.85f : 0.3f) : (a.windows[x].n_gates < 24 ? 1.0f : 0.7f);
+    return choose_layout(n, g, fill, grp.nblk, WARPS, SB::R, room);
+  };
   auto dest_bins = [&](u32 set, const Layout& l) {
-    Dest<W> d;
-    d.dense = false;
+    Dest d;
+    d.dense = 0;
     d.l = l;
     d.keys = a.bin_keys[set & 1];
     d.coeffs = a.bin_coeffs[set & 1];
@@ -620,16 +1017,15 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, S& s)
     d.fail = &bs->fail[set % 3];
     return d;
   };
-  auto rows_per_bin = [&] {
-    return (u32)((float)S::R / fminf(fmaxf(1.5f, 1.15f * rho), 3.0f));
-  };
-  // `ph` counts buffer fills: set ph lives in buffer ph & 1, counters ph % 3.
   if (!resumed) {
     // Deal the dense rows into the bins of the first window.
-    const WinDesc w = a.windows[win];
-    lay = choose_layout(N, rows_per_bin(), grp.nblk, a.room[0]);
-    load_grouping<W>(s, a, w);
-    const Dest<W> d = dest_bins(0, lay);
+    lay = layout_for((float)N, win, a.room[0]);
+    if (tid == 0) {
+      v.wn = a.windows[win];
+      v.d = dest_bins(0, lay);
+    }
+    __syncthreads();
+    load_grouping<W>(v, a);
     for (u64 r0 = (u64)grp.bid * T; r0 < N; r0 += (u64)grp.nblk * T) {
       const u64 r = r0 + tid;
       u64 k[W];
@@ -640,7 +1036,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, S& s)
         c = __ldcg(a.coeffs + r);
         h = lin_hash<W>(k, a.lin);
       }
-      put_row<W, ALG>(s, d, k, c, h, r < N, gates, w);
+      put_row<W, ALG>(v, k, c, h, r < N, gates);
     }
     grid_barrier(st, gen, grp);
     if (*(volatile u32*)&st->error) return;
@@ -655,238 +1051,94 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, S& s)
     }
   }
 
+  Layout prev{0, 0, 0};  // of the counters to clear
   for (;;) {
-    const WinDesc w = a.windows[win];
+    const float grow = next_grow;
     const bool last = win + 1 >= a.n_windows;
-    const WinDesc wn = last ? WinDesc{} : a.windows[win + 1];
-    const u32 set = ph, nset = ph + 1;
-    const u32* cnt = a.counts + (u64)(set % 3) * a.count_words;
-    const u64* bk = a.bin_keys[set & 1];
-    const double* bc = a.bin_coeffs[set & 1];
-    const u32* bh = a.bin_hash[set & 1];
-    const u32* bsp = a.spill_bin[set & 1];
-    const u64 spill0 = (u64)lay.bins * lay.cap;
-    Dest<W> d;
-    Layout nlay = lay;
-    if (last) {
-      d = Dest<W>{};
-      d.dense = true;
-      d.keys = a.keys;
-      d.coeffs = a.coeffs;
-      d.room = a.dense_room;
-      d.n_dense = &bs->n_dense;
-      d.fail = &bs->fail[nset % 3];
-    } else {
-      nlay = choose_layout(w.noise == 2 ? N : N + N / 2, rows_per_bin(), grp.nblk, a.room[nset & 1]);
-      d = dest_bins(nset, nlay);
-      load_grouping<W>(s, a, wn);
+    const u32 set = ph % 3, nset = (ph + 1) % 3;
+    // The rows that will leave this window: as many more or fewer as left the
+    // earlier one like it; without one, a reclaim mostly undoes the growth.
+    const float* h = alike((float)N, win);
+    const float ratio = h ? __ldcg(h + 1) : (a.windows[win].noise == 2 ? 1.0f : 1.5f);
+    const Layout nlay = last ? lay : layout_for((float)N * ratio, win + 1, a.room[(ph + 1) & 1]);
+    if (tid == 0) {
+      v.w = a.windows[win];
+      v.wn = last ? WinDesc{} : a.windows[win + 1];
+      if (last) {
+        Dest d{};
+        d.dense = 1;
+        d.keys = a.keys;
+        d.coeffs = a.coeffs;
+        d.room = a.dense_room;
+        d.n_dense = &bs->n_dense;
+        d.fail = &bs->fail[nset];
+        v.d = d;
+      } else {
+        v.d = dest_bins(ph + 1, nlay);
+      }
+      v.bk = a.bin_keys[ph & 1];
+      v.bc = a.bin_coeffs[ph & 1];
+      v.bh = a.bin_hash[ph & 1];
+      v.bsp = a.spill_bin[ph & 1];
+      v.cnt = a.counts + (u64)set * a.count_words;
+      v.lay = lay;
+      v.first = first;
+      v.grow = grow;
+      v.spilled = *(volatile u32*)&bs->n_spill[set];
+      v.kept = v.n_defer = 0;
     }
-    const u32 G = w.n_gates;
-    for (u32 i = tid; i < WIN_MAX; i += T) s.born_all[i] = s.anti_all[i] = 0;
-    if (tid == 0) s.kept = 0;
-    const u32 spilled = *(volatile u32*)&bs->n_spill[set % 3];
-    const double* factors = a.tables + (u64)w.table * a.table_len;
-    const u32 lastw = a.table_len ? a.table_len - 1 : 0;
-    BinRules R;
-    R.n_units = a.n_units;
-    R.minc = a.min_coeff;
-    R.wcut = a.max_weight;
-    R.ccut = a.has_min_coeff != 0;
-
-    // A finished row: the reclaim after the window, then its next bin.
-    u32 kept = 0;
-    auto finish_row = [&](u64* k, double c, u32 h, bool act) {
-      if (act && w.noise) {
-        const u32 wt = Ops::template weight<W>(k, a.n_units);
-        c = __dmul_rn(c, __ldg(factors + (wt < lastw ? wt : lastw)));
-        if (w.noise == 2)
-          act = (a.max_weight == NO_WEIGHT_CUT || wt <= a.max_weight) && (!a.has_min_coeff || fabs(c) >= a.min_coeff);
-      }
-      kept += act;
-      put_row<W, ALG>(s, d, k, c, h, act, gates, wn);
-    };
-
-    const bool dynamic = lay.bins > grp.nblk;
-    u32 bin = grp.bid, depth0 = 0;
+    for (u32 i = tid; i < WIN_MAX; i += T) v.born_all[i] = v.anti_all[i] = 0;
     __syncthreads();
-    for (;;) {
-      if (dynamic) {
-        if (tid == 0) s.tick = atomicAdd(&bs->ticket[set % 3], 1u);
-        __syncthreads();
-        bin = s.tick;
+    load_grouping<W>(v, a);
+
+    u32 kept = 0, depth0 = 0;
+    if (lay.bins == grp.nblk * WARPS) {  // a bin a warp
+      const u32 bin = grp.bid * WARPS + (tid >> 5);
+      u32 unused = 0;
+      if (!run_bin<W, ALG>(a, v, sw[tid >> 5], bin, unused, kept) && lane == 0) v.defer[atomicAdd(&v.n_defer, 1u)] = bin;
+      __syncthreads();
+      const u32 nd = v.n_defer;
+      for (u32 i = 0; i < nd; ++i) {
+        run_bin<W, ALG>(a, v, sb, v.defer[i], depth0, kept);
         __syncthreads();
       }
-      if (bin >= lay.bins) break;
-      const u32 n_all = __ldcg(cnt + (u64)bin * lay.stride);
-      const u32 n_bin = n_all < lay.cap ? n_all : lay.cap;
-      const bool has_spill = n_all > lay.cap;
-      const u64 row0 = (u64)bin * lay.cap;
-      if (G == 0 || first >= G) {
-        // no rotation: straight through
-        for (u32 r0 = 0; r0 < n_bin; r0 += T) {
-          const u32 r = r0 + tid;
-          u64 k[W];
-          double c = 0.0;
-          u32 h = 0;
-          if (r < n_bin) {
-            load_key<W>(bk, row0 + r, k);
-            c = __ldcg(bc + row0 + r);
-            h = __ldcg(bh + row0 + r);
-          }
-          finish_row(k, c, h, r < n_bin);
-        }
-        for (u32 r0 = 0; has_spill && r0 < spilled; r0 += T) {
-          const u32 r = r0 + tid;
-          const bool mine = r < spilled && __ldcg(bsp + r) == bin;
-          u64 k[W];
-          double c = 0.0;
-          u32 h = 0;
-          if (mine) {
-            load_key<W>(bk, spill0 + r, k);
-            c = __ldcg(bc + spill0 + r);
-            h = __ldcg(bh + spill0 + r);
-          }
-          finish_row(k, c, h, mine);
-        }
-      } else if (n_all) {
-        // Parts of the bin: `part` of 2^depth by split_bits, in order.
-        u32 depth = depth0, part = 0;
-        while (depth < 24 && (n_all >> depth) > (u32)S::R * 7 / 8) ++depth;
-        const u32 base = depth;
-        for (;;) {
-          for (u32 i = tid; i < G; i += T) s.born[i] = s.anti[i] = 0;
-          for (int i = tid; i < S::SLOTS / 4; i += T)
-            reinterpret_cast<uint4*>(s.tab)[i] = make_uint4(TAB_EMPTY, TAB_EMPTY, TAB_EMPTY, TAB_EMPTY);
-          if (tid == 0) s.n = s.n_list[0] = s.n_list[1] = 0;
-          if (fetcher) {
-            for (u32 g = first; g < first + 2 && g < G; ++g) fetch_gate<W>(&s.gate[g & 3], gates + w.gate + g);
-            cp_async_wait();
-          }
+    } else {
+      const bool dynamic = lay.bins > grp.nblk;
+      u32 bin = grp.bid;
+      for (;;) {
+        if (dynamic) {
+          if (tid == 0) v.tick = atomicAdd(&bs->ticket[set], 1u);
           __syncthreads();
-          u32 n = n_all;
-          const bool whole = depth == 0 && !has_spill;
-          if (whole) {
-            for (u32 r = tid; r < n_bin; r += T) {
-              u64 k[W];
-              load_key<W>(bk, row0 + r, k);
-              const double c = __ldcg(bc + row0 + r);
-              const u32 h = __ldcg(bh + row0 + r);
-#pragma unroll
-              for (int x = 0; x < W; ++x) s.key[x][r] = k[x];
-              s.coef[r] = c;
-              s.h[r] = h;
-              tab_insert(s, h, r, tab_start<S>(h));
-            }
-          } else {
-            auto take = [&](u64 src) {
-              u64 k[W];
-              load_key<W>(bk, src, k);
-              const u32 h = __ldcg(bh + src);
-              if (depth && (split_bits(group_hash_list<W, ALG>(k, h, a, w)) >> (32 - depth)) != part) return;
-              const u32 r = atomicAdd(&s.n, 1u);
-              if (r >= (u32)S::R) return;
-#pragma unroll
-              for (int x = 0; x < W; ++x) s.key[x][r] = k[x];
-              s.coef[r] = __ldcg(bc + src);
-              s.h[r] = h;
-              tab_insert(s, h, r, tab_start<S>(h));
-            };
-            for (u32 r = tid; r < n_bin; r += T) take(row0 + r);
-            if (has_spill)
-              for (u32 r = tid; r < spilled; r += T)
-                if (__ldcg(bsp + r) == bin) take(spill0 + r);
-            __syncthreads();
-            n = s.n;
-          }
-          bool fits = n <= (u32)S::R;
-          for (u32 g = first; fits && g < G; ++g) {
-            if (fetcher) cp_async_wait_1();
-            __syncthreads();
-            if (g > first) {
-              n += s.born[g - 1];
-              if (n > (u32)S::R) {
-                fits = false;
-                break;
-              }
-            }
-            if (fetcher) {
-              if (g + 2 < G) fetch_gate<W>(&s.gate[(g + 2) & 3], gates + w.gate + g + 2);
-              cp_async_commit();
-            }
-            rotate_rows<W, ALG>(s, s.gate[g & 3], R, n, g & 1, &s.born[g], &s.anti[g]);
-          }
-          if (fetcher) cp_async_wait();
+          bin = v.tick;
           __syncthreads();
-          if (fits) {
-            n += s.born[G - 1];
-            fits = n <= (u32)S::R;
-          }
-          if (!fits) {  // run the part again in halves
-            ++depth;
-            part <<= 1;
-            if (depth0 < depth && depth0 < 8) depth0 = depth;
-            if (depth > 24) {
-              if (tid == 0) atomicOr(&st->error, ERR_CAPACITY);
-              break;
-            }
-            __syncthreads();
-            continue;
-          }
-          for (u32 i = tid; i < G; i += T) {
-            s.born_all[i] += s.born[i];
-            s.anti_all[i] += s.anti[i];
-          }
-          for (u32 r0 = 0; r0 < n; r0 += T) {
-            const u32 r = r0 + tid;
-            u64 k[W];
-            double c = 0.0;
-            u32 h = 0;
-            if (r < n) {
-#pragma unroll
-              for (int x = 0; x < W; ++x) k[x] = s.key[x][r];
-              c = s.coef[r];
-              h = s.h[r];
-            }
-            finish_row(k, c, h, r < n);
-          }
-          __syncthreads();
-          while (depth && (part & 1u)) {
-            part >>= 1;
-            --depth;
-          }
-          if (!depth) break;
-          ++part;
-          while (depth < base) {
-            ++depth;
-            part <<= 1;
-          }
         }
+        if (bin >= lay.bins) break;
+        run_bin<W, ALG>(a, v, sb, bin, depth0, kept);
+        __syncthreads();
+        if (!dynamic) break;
       }
-      if (!dynamic) break;
     }
     // Block totals: rows kept, rows created and rows branching per rotation.
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) kept += __shfl_xor_sync(FULL, kept, o);
-    if (lane == 0 && kept) atomicAdd(&s.kept, kept);
+    if (lane == 0 && kept) atomicAdd(&v.kept, kept);
     __syncthreads();
-    if (tid == 0 && s.kept) atomicAdd(&bs->n[nset % 3], (u64)s.kept);
-    for (u32 i = tid; i < G; i += T) {
-      if (s.born_all[i]) {
-        atomicAdd(a.born + w.op + i, s.born_all[i]);
-        atomicAdd(&bs->grown[nset % 3], (u64)s.born_all[i]);
+    if (tid == 0 && v.kept) atomicAdd(&bs->n[nset], (u64)v.kept);
+    for (u32 i = tid; i < v.w.n_gates; i += T) {
+      if (v.born_all[i]) {
+        atomicAdd(a.born + v.w.op + i, v.born_all[i]);
+        atomicAdd(&bs->grown[nset], (u64)v.born_all[i]);
       }
-      if (s.anti_all[i]) atomicAdd(a.anti + w.op + i, (u64)s.anti_all[i]);
+      if (v.anti_all[i]) atomicAdd(a.anti + v.w.op + i, (u64)v.anti_all[i]);
     }
     // The counter set after next: its last readers ran the window before this one.
     if (ph > a.phase0) {
-      u32* z = a.counts + (u64)((ph + 2) % 3) * a.count_words;
-      const Layout pl{s.x[6], s.x[7], 0};
-      for (u32 b = grp.bid * T + tid; b < pl.bins; b += grp.nblk * T) z[(u64)b * pl.stride] = 0;
+      const u32 z = (ph + 2) % 3;
+      u32* zc = a.counts + (u64)z * a.count_words;
+      for (u32 b = grp.bid * T + tid; b < prev.bins; b += grp.nblk * T) zc[(u64)b * prev.stride] = 0;
       if (grp.bid == 0 && tid == 0) {
-        bs->n[(ph + 2) % 3] = 0;
-        bs->grown[(ph + 2) % 3] = 0;
-        bs->n_spill[(ph + 2) % 3] = 0;
-        bs->ticket[(ph + 2) % 3] = 0;
+        bs->n[z] = bs->grown[z] = 0;
+        bs->n_spill[z] = bs->ticket[z] = 0;
       }
     }
     __syncthreads();
@@ -894,49 +1146,52 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, S& s)
       if (barrier_arrive(st, grp)) barrier_release(st, gen);
       else barrier_wait(st, gen);
       ++gen;
-      const u64 nn = ld_volatile(&bs->n[nset % 3]), gr = ld_volatile(&bs->grown[nset % 3]);
-      const u32 e = *(volatile u32*)&st->error, f = *(volatile u32*)&bs->fail[nset % 3];
-      s.y[0] = nn;
-      s.y[1] = gr;
-      s.x[0] = e;
-      s.x[1] = f;
-      s.x[6] = lay.bins;
-      s.x[7] = lay.stride;
+      const u64 nn = ld_volatile(&bs->n[nset]), gr = ld_volatile(&bs->grown[nset]);
+      const u32 e = *(volatile u32*)&st->error, f = *(volatile u32*)&bs->fail[nset];
+      v.y[0] = nn;
+      v.y[1] = gr;
+      v.x[0] = e;
+      v.x[1] = f;
     }
     __syncthreads();
-    if (s.x[0]) return;
-    if (s.x[1]) {  // the next buffer was too small: this window is run again after the host has grown it
+    if (v.x[0]) return;
+    if (v.x[1]) {  // the next buffer was too small: this window is run again after the host has grown it
       if (grp.bid == 0 && tid == 0) {
         bs->stopped = 1;
         bs->dense_start = 0;
-        bs->op = w.op + first;
+        bs->op = v.w.op + first;
         bs->rows = N;
         bs->phase = ph;
         bs->bins = lay.bins;
         bs->stride = lay.stride;
         bs->cap = lay.cap;
         bs->rho = rho;
+        bs->grow = grow;
       }
       return;
     }
-    const u64 nn = s.y[0];
+    const u64 nn = v.y[0];
     if (grp.bid == 0 && tid == 0) {
-      if (w.noise) a.hist[w.op + G] = nn;
-      u64 t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      a.stamps[w.op_end - 1] = t;
+      if (v.w.noise) a.hist[v.w.op + v.w.n_gates] = nn;
+      stamp_op(a.stamps, v.w.op_end - 1);
+      if (N && !first) {  // read by windows at least 3 further on
+        a.growth[3 * win] = (float)(N + v.y[1]) / (float)N;
+        a.growth[3 * win + 1] = (float)nn / (float)N;
+        a.growth[3 * win + 2] = (float)N;
+      }
     }
-    const float g = N ? (float)(N + s.y[1]) / (float)N : 1.0f;
-    rho = fmaxf(g, 0.85f * rho);
+    rho = fmaxf(N ? (float)(N + v.y[1]) / (float)N : 1.0f, 0.85f * rho);
     N = nn;
+    prev = lay;
     lay = nlay;
     first = 0;
     ++ph;
     ++win;
     if (win >= a.n_windows) break;
+    __syncthreads();  // v is rewritten
   }
   if (grp.bid == 0 && tid == 0) {
     st->n[0] = N;
-    st->end_op = a.windows[a.n_windows - 1].op_end;
+    st->end_op = a.op_end;
   }
 }

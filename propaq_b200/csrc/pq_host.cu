@@ -270,6 +270,7 @@ struct Slot {
   u32* counts = nullptr;
   pq::BinState* bin_state = nullptr;
   pq::WinDesc* d_windows = nullptr;
+  float* growth = nullptr;  // three words per window (BinArgs::growth), behind bin_state
   size_t windows_cap = 0;
   pq::BasisDesc* d_basis = nullptr;
   size_t basis_cap = 0;
@@ -327,6 +328,7 @@ struct Slot {
     bin_state = nullptr;
     d_windows = nullptr;
     d_basis = nullptr;
+    growth = nullptr;
     windows_cap = basis_cap = 0;
     for (void* p : {(void*)d_gates, (void*)d_tables, (void*)partials, (void*)frame_img, (void*)frame_sgn,
                     (void*)host_state, (void*)host_factor, (void*)host_keep})
@@ -415,6 +417,7 @@ struct pq_engine {
   // default-sized gradient needed to record every op.
   DevBuf g_pool, g_lam, g_ops;
   u32* d_lin = nullptr;  // linear hash tables of the binned sweep
+  pq::BinState* h_bins = nullptr;  // pinned
   DevBuf sort_buf;  // radix-sort scratch and sorted rows (observable folding, sorted term output)
   std::vector<DevBuf> g_ck;
   size_t g_need = 0;
@@ -459,7 +462,7 @@ struct pq_engine {
     for (DevBuf& b : g_ck) b.release();
     for (void* p : {(void*)d_states, (void*)d_args, (void*)d_block_inst, (void*)d_err, (void*)d_idle, (void*)d_lin})
       if (p) dfree(p);
-    for (void* p : {(void*)h_states, (void*)h_args, (void*)h_block_inst})
+    for (void* p : {(void*)h_states, (void*)h_args, (void*)h_block_inst, (void*)h_bins})
       if (p) cudaFreeHost(p);
     for (auto ev : {ev_begin, ev_end, ev_l0, ev_l1})
       if (ev) cudaEventDestroy(ev);
@@ -1253,6 +1256,7 @@ void plan_windows(Plan& P) {
   std::vector<std::vector<u64>> span;
   std::vector<int> pivot;
   std::vector<u64> used(W), g(W);
+  std::unordered_map<u64, std::vector<u32>> seen;  // windows by their generators
   for (size_t i = 0; i < no;) {
     pq::WinDesc w{};
     w.op = (u32)i;
@@ -1304,6 +1308,11 @@ void plan_windows(Plan& P) {
       }
       w.gate = P.ops[i].idx;
       w.n_gates = (u32)len;
+      w.commute = 1;
+      if (!w.disjoint)
+        for (size_t x = 1; x < len && w.commute; ++x)
+          for (size_t y = 0; y < x && w.commute; ++y)
+            if (host_anticommutes(P.alg, W, gen(i + x), gen(i + y))) w.commute = 0;
       i += len;
     }
     w.n_basis = (u32)P.basis.size() - w.basis;
@@ -1334,6 +1343,20 @@ void plan_windows(Plan& P) {
       ++i;
     }
     w.op_end = (u32)i;
+    // the last window of the same generators and angles' kind, as Trotter
+    // steps repeat them
+    w.like = 0xffffffffu;
+    u64 sig = w.n_gates * 4 + w.noise;
+    for (u32 k = 0; k < w.n_gates; ++k)
+      for (int x = 0; x < W; ++x) sig = (sig ^ gen(w.op + k)[x]) * 0x9E3779B97F4A7C15ULL ^ (sig >> 29);
+    std::vector<u32>& same = seen[sig];
+    const u32 self = (u32)P.windows.size();
+    for (size_t k = same.size(); k-- > 0;)
+      if (same[k] + 4 <= self) {
+        w.like = same[k];
+        break;
+      }
+    same.push_back(self);
     P.windows.push_back(w);
   }
 }
@@ -1479,12 +1502,20 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
   }
   if (!S.counts && (e = dmalloc(&S.counts, 3 * (size_t)pq::COUNT_WORDS * 4)) != cudaSuccess)
     return E->cuda_fail(e, "bin counters");
-  if (!S.bin_state && (e = dmalloc(&S.bin_state, sizeof(pq::BinState))) != cudaSuccess)
-    return E->cuda_fail(e, "bin state");
-  if ((e = grow_pair<pq::WinDesc>(&S.d_windows, nullptr, &S.windows_cap, std::max<size_t>(P.windows.size(), 1))) !=
-          cudaSuccess ||
-      (e = grow_pair<pq::BasisDesc>(&S.d_basis, nullptr, &S.basis_cap, std::max<size_t>(P.basis.size(), 1))) !=
-          cudaSuccess)
+  const size_t nw = std::max<size_t>(P.windows.size(), 1);
+  if (S.windows_cap < nw) {  // windows, and the state with the growth table behind it
+    if (S.bin_state) dfree(S.bin_state);
+    S.bin_state = nullptr;
+    if ((e = grow_pair<pq::WinDesc>(&S.d_windows, nullptr, &S.windows_cap, nw)) != cudaSuccess ||
+        (e = dmalloc(reinterpret_cast<char**>(&S.bin_state), sizeof(pq::BinState) + 3 * nw * sizeof(float))) !=
+            cudaSuccess) {
+      S.windows_cap = 0;
+      return E->cuda_fail(e, "windows");
+    }
+    S.growth = reinterpret_cast<float*>(S.bin_state + 1);
+  }
+  if ((e = grow_pair<pq::BasisDesc>(&S.d_basis, nullptr, &S.basis_cap, std::max<size_t>(P.basis.size(), 1))) !=
+      cudaSuccess)
     return E->cuda_fail(e, "windows");
   for (int i = 0; i < 2; ++i)
     if (int rc = E->ensure_bins(S, i, std::max(ROOM, S.bin_W[i] == W ? S.room[i] : 0), W)) return rc;
@@ -1499,7 +1530,7 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     cudaMemsetAsync(S.stamps, 0, no * 8, E->stream);
   }
   cudaMemsetAsync(S.counts, 0, 3 * (size_t)pq::COUNT_WORDS * 4, E->stream);
-  cudaMemsetAsync(S.bin_state, 0, sizeof(pq::BinState), E->stream);
+  cudaMemsetAsync(S.bin_state, 0, sizeof(pq::BinState) + 3 * nw * sizeof(float), E->stream);
   pq::BinArgs a{};
   a.ops = S.d_ops;
   a.gates = S.d_gates;
@@ -1519,6 +1550,7 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
   a.n0 = P.n0;
   a.counts = S.counts;
   a.count_words = pq::COUNT_WORDS;
+  a.growth = S.growth;
   a.born = S.tickets;
   a.anti = S.anti;
   a.hist = S.hist;
@@ -1529,7 +1561,9 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
   a.hold_us = std::min<u32>(E->lim.hold_us, 100000);
   const int grid = with_bins(W, P.alg, [](auto w, auto alg) { return pq::bins_grid<w, alg>(); });
   if (grid <= 0) return E->fail(PQ_ERR_CUDA, "the binned sweep does not fit this device");
-  pq::BinState hb{};
+  if (!E->h_bins && (e = cudaMallocHost(&E->h_bins, sizeof(pq::BinState))) != cudaSuccess)
+    return E->cuda_fail(e, "bin state");
+  pq::BinState& hb = *E->h_bins;
   for (bool first = true;; first = false) {
     for (int i = 0; i < 2; ++i) {
       a.bin_keys[i] = S.bin_keys[i];

@@ -1376,20 +1376,39 @@ struct BinSize {
   static constexpr int T = 256;
   static constexpr int BLOCKS = 2;  // per SM
   static constexpr int GRID_R = W == 1 ? 3328 : (W == 2 ? 2560 : (W == 4 ? 2048 : 1152));
-  static constexpr int SOLO_R = W == 1 ? 7168 : 2 * GRID_R;
+  static constexpr int WARP_R = W <= 4 ? 128 : 120;
+  static constexpr int SOLO_WARP_R = 128;  // up to 64 rows: two rounds of 32 at the most
+  // solo up to 1,024 rows: beyond, a rotation takes the block 1.5 us and more,
+  // a grid window of a dozen rotations 17 us
+  static constexpr int SOLO_R = 2048;
+  using Warp = BinSmem<W, 32, WARP_R, 512>;
   using Grid = BinSmem<W, T, GRID_R, (W <= 2 ? 8192 : 4096)>;
-  using Solo = BinSmem<W, T, SOLO_R, (W <= 2 ? 16384 : 8192)>;
+  using SoloWarp = BinSmem<W, 32, SOLO_WARP_R, 512>;
+  using Solo = BinSmem<W, T, SOLO_R, 4096>;
+  struct GridSmem {
+    union Rows {
+      Grid block;
+      Warp warp[T / 32];
+    } rows;
+    WinSmem<W> win;
+  };
+  union SoloSmem {
+    Solo block;
+    SoloWarp warp;
+  };
 };
 
 template <int W, int ALG>
-__global__ void __launch_bounds__(BinSize<W>::T, 1) solo_kernel(const BinArgs a) {
+__global__ void __launch_bounds__(BinSize<W>::T, 1) solo_kernel(const __grid_constant__ BinArgs a) {
   extern __shared__ __align__(16) unsigned char bin_smem[];
-  solo_body<W, ALG>(a, *reinterpret_cast<typename BinSize<W>::Solo*>(bin_smem));
+  auto& s = *reinterpret_cast<typename BinSize<W>::SoloSmem*>(bin_smem);
+  solo_body<W, ALG>(a, s.warp, s.block);
 }
 template <int W, int ALG>
-__global__ void __launch_bounds__(BinSize<W>::T, BinSize<W>::BLOCKS) bins_kernel(const BinArgs a) {
+__global__ void __launch_bounds__(BinSize<W>::T, BinSize<W>::BLOCKS) bins_kernel(const __grid_constant__ BinArgs a) {
   extern __shared__ __align__(16) unsigned char bin_smem[];
-  bins_body<W, ALG>(a, Grp{blockIdx.x, gridDim.x}, *reinterpret_cast<typename BinSize<W>::Grid*>(bin_smem));
+  auto& s = *reinterpret_cast<typename BinSize<W>::GridSmem*>(bin_smem);
+  bins_body<W, ALG>(a, Grp{blockIdx.x, gridDim.x}, s.win, s.rows.block, s.rows.warp);
 }
 
 // A batch: each instance owns the contiguous blocks [blk_begin, blk_begin +
@@ -1795,35 +1814,37 @@ cudaError_t launch_sweep(const SweepArgs& a, int grid, cudaStream_t s, int build
 
 template <int W, int ALG>
 cudaError_t launch_solo(const BinArgs& a, cudaStream_t s) {
-  using S = typename BinSize<W>::Solo;
+  using S = typename BinSize<W>::SoloSmem;
   static_assert(sizeof(S) <= 227 * 1024, "solo shared memory");
   if (cudaError_t e = cudaFuncSetAttribute(solo_kernel<W, ALG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)sizeof(S)))
     return e;
-  solo_kernel<W, ALG><<<1, S::T, sizeof(S), s>>>(a);
+  solo_kernel<W, ALG><<<1, BinSize<W>::T, sizeof(S), s>>>(a);
   return cudaGetLastError();
 }
 
 template <int W, int ALG>
 int bins_grid() {
-  using S = typename BinSize<W>::Grid;
+  using S = typename BinSize<W>::GridSmem;
   static_assert(BinSize<W>::BLOCKS * (sizeof(S) + 1024) <= 228 * 1024, "resident blocks");
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (cudaFuncSetAttribute(bins_kernel<W, ALG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(S)) !=
           cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bins_kernel<W, ALG>, S::T, sizeof(S)) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bins_kernel<W, ALG>, BinSize<W>::T, sizeof(S)) !=
+          cudaSuccess)
     return 0;
   return sms * per;
 }
 
 template <int W, int ALG>
 cudaError_t launch_bins(const BinArgs& a, int grid, cudaStream_t s) {
-  using S = typename BinSize<W>::Grid;
+  using S = typename BinSize<W>::GridSmem;
   BinArgs args = a;
   void* params[] = {&args};
-  return cudaLaunchCooperativeKernel((const void*)bins_kernel<W, ALG>, dim3(grid), dim3(S::T), params, sizeof(S), s);
+  return cudaLaunchCooperativeKernel((const void*)bins_kernel<W, ALG>, dim3(grid), dim3(BinSize<W>::T), params,
+                                     sizeof(S), s);
 }
 
 template <int W, int ALG>

@@ -170,6 +170,9 @@ struct WinDesc {
   u32 noise, table;    // 0 none, 1 scale, 2 scale and reclaim; its noise table
   u32 basis, n_basis;  // grouping: BasisDescs
   u32 disjoint;        // a basis vector counts only where its rotation anticommutes
+  u32 commute;         // its generators commute pairwise
+  u32 like;            // an earlier window of the same rotations (at least 4 back), or 0xffffffff
+  u32 pad_;
 };
 struct BasisDesc {
   u32 bit;   // pivot key bit, in no other vector of the window's basis
@@ -191,7 +194,7 @@ struct BinState {
   u32 op, phase;   // first op not run; count of buffer fills so far
   u64 rows;
   u32 bins, stride, cap;
-  float rho;
+  float rho, grow;
 };
 
 struct BinArgs {
@@ -204,7 +207,6 @@ struct BinArgs {
   u32 n_gdesc, n_windows;
   u32 table_len, n_units;
   u32 op_begin, op_end;
-  u32 first_gate, pad_;  // gate descriptor of the first rotation from op_begin on
   u32 max_weight, has_min_coeff;
   double min_coeff;
   u64 n0;             // dense rows at entry
@@ -219,6 +221,8 @@ struct BinArgs {
   u32* counts;        // three sets of COUNT_WORDS
   u32 count_words;
   u32 resume, phase0; // continue a stopped sweep from BinState
+  float* growth;      // per window: growth of the live count inside it, rows leaving / entering,
+                      // rows entering (0: not run on the grid)
   u32* born;          // per op: rows created
   u64* anti;          // per op: rows anticommuting
   u64* hist;          // noise ops: live count after

@@ -2,8 +2,10 @@
 case against the oracle: live count after every rotation, term set, every
 coefficient bit for bit, terms below the cutoff, expectation value.
 
-* observables around the rows one block holds (solo runs, and the hand-over
-  to the grid) for 1-, 2-, 4- and 8-word keys;
+* observables around the rows one warp and one block hold (solo runs, and the
+  hand-over to the grid) for 1-, 2-, 4- and 8-word keys;
+* live sets of a few rows per warp, and on either side of the line between
+  bins of warps and bins of blocks;
 * groups as large as a window's span allows (dense cosets), and more rows than
   the bins hold, so that bins are split;
 * buffers that grow mid-run on a fresh engine, final rows included;
@@ -47,10 +49,9 @@ def observable(n, n_terms, W, seed):
     return arr, rng.normal(size=n_terms)
 
 
-@pytest.mark.parametrize("n,solo", [(24, 7168), (60, 5120), (120, 4096), (250, 2304)], ids=["W1", "W2", "W4", "W8"])
-@pytest.mark.parametrize("where", ["below", "at", "above", "full"])
-def test_rows_around_one_block(gpu_engine, oracle, n, solo, where):
-    n0 = {"below": solo // 2 - 1, "at": solo // 2, "above": solo // 2 + 1, "full": solo + 3}[where]
+@pytest.mark.parametrize("n", [24, 60, 120, 250], ids=["W1", "W2", "W4", "W8"])
+@pytest.mark.parametrize("n0", [63, 64, 65, 1023, 1024, 1025, 2051, 7171, 40000])
+def test_rows_around_one_unit(gpu_engine, oracle, n, n0):
     base = random_pauli_problem(n, n, n_gates=24, max_weight=6, min_coeff=1e-3)
     keys, coeffs = observable(n, n0, base.n_words, n0)
     p = Problem(0, n, base.n_words, keys, coeffs, base.gate_keys, base.angles, base.offsets, base.diag, 6, 1e-3)
