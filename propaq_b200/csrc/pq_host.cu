@@ -265,8 +265,8 @@ struct Slot {
   double* bin_coeffs[2] = {nullptr, nullptr};
   u32* bin_hash[2] = {nullptr, nullptr};
   u32* spill_bin[2] = {nullptr, nullptr};
-  u64 room[2] = {0, 0};
-  int bin_W[2] = {0, 0};
+  u64 room[2] = {0, 0};  // rows they hold at the width of the run (ensure_bins)
+  u64 bin_rows[2] = {0, 0}, bin_words[2] = {0, 0};  // rows and key words allocated
   u32* counts = nullptr;
   pq::BinState* bin_state = nullptr;
   pq::WinDesc* d_windows = nullptr;
@@ -313,8 +313,7 @@ struct Slot {
     bin_keys[i] = nullptr;
     bin_coeffs[i] = nullptr;
     bin_hash[i] = spill_bin[i] = nullptr;
-    room[i] = 0;
-    bin_W[i] = 0;
+    room[i] = bin_rows[i] = bin_words[i] = 0;
   }
   void free_all() {
     free_rows();
@@ -418,6 +417,7 @@ struct pq_engine {
   DevBuf g_pool, g_lam, g_ops;
   u32* d_lin = nullptr;  // linear hash tables of the binned sweep
   pq::BinState* h_bins = nullptr;  // pinned
+  DevBuf batch_args;  // arguments of a binned batch's solo runs
   DevBuf sort_buf;  // radix-sort scratch and sorted rows (observable folding, sorted term output)
   std::vector<DevBuf> g_ck;
   size_t g_need = 0;
@@ -458,7 +458,7 @@ struct pq_engine {
   ~pq_engine() {
     if (stream) cudaStreamSynchronize(stream);
     for (auto& s : slots) s.free_all();
-    for (DevBuf* b : {&g_pool, &g_lam, &g_ops, &sort_buf}) b->release();
+    for (DevBuf* b : {&g_pool, &g_lam, &g_ops, &sort_buf, &batch_args}) b->release();
     for (DevBuf& b : g_ck) b.release();
     for (void* p : {(void*)d_states, (void*)d_args, (void*)d_block_inst, (void*)d_err, (void*)d_idle, (void*)d_lin})
       if (p) dfree(p);
@@ -566,20 +566,23 @@ struct pq_engine {
     return PQ_OK;
   }
   // A bin buffer of at least `rows` rows of Wn words; its contents are lost
-  // when it is replaced.
+  // when it is replaced.  Slot 0's buffers serve every slot: an engine runs
+  // one binned sweep at a time.
   int ensure_bins(Slot& S, int i, u64 rows, int Wn) {
-    if (S.bin_W[i] == Wn && S.room[i] >= rows) return PQ_OK;
-    S.free_bins(i);
-    cudaError_t e;
-    if ((e = dmalloc(&S.bin_keys[i], rows * Wn * 8)) != cudaSuccess ||
-        (e = dmalloc(&S.bin_coeffs[i], rows * 8)) != cudaSuccess ||
-        (e = dmalloc(&S.bin_hash[i], rows * 4)) != cudaSuccess ||
-        (e = dmalloc(&S.spill_bin[i], rows / 8 * 4)) != cudaSuccess) {
+    if (S.bin_rows[i] < rows || S.bin_words[i] < rows * Wn) {
+      const u64 nr = std::max(rows, S.bin_rows[i]), nw = std::max(rows * Wn, S.bin_words[i]);
       S.free_bins(i);
-      return cuda_fail(e, "allocating bins");
+      cudaError_t e;
+      if ((e = dmalloc(&S.bin_keys[i], nw * 8)) != cudaSuccess || (e = dmalloc(&S.bin_coeffs[i], nr * 8)) != cudaSuccess ||
+          (e = dmalloc(&S.bin_hash[i], nr * 4)) != cudaSuccess ||
+          (e = dmalloc(&S.spill_bin[i], nr / 8 * 4)) != cudaSuccess) {
+        S.free_bins(i);
+        return cuda_fail(e, "allocating bins");
+      }
+      S.bin_rows[i] = nr;
+      S.bin_words[i] = nw;
     }
-    S.room[i] = rows;
-    S.bin_W[i] = Wn;
+    S.room[i] = std::min(S.bin_rows[i], S.bin_words[i] / Wn);
     return PQ_OK;
   }
   int rebuild_table(Slot& S, u64 n) {
@@ -1488,19 +1491,19 @@ int execute_launches(pq_engine* E, Slot& S, Plan& P, int grid, bool* began, size
   return PQ_OK;
 }
 
-// Runs every op of a plan on the binned sweep: one block alone while the rows
-// fit it, then the windows on the whole grid; a buffer that turned out too
-// small is grown and the sweep goes on from the window that needed it.
-int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
+// The buffers and arguments of a plan's binned sweep, its inputs enqueued;
+// `st` is its sweep state on the device.
+int prepare_bins(pq_engine* E, Slot& S, Plan& P, pq::SweepState* st, pq::BinArgs* out) {
   cudaError_t e;
   const int W = P.W;
   const size_t no = P.ops.size();
   constexpr u64 ROOM = 1ULL << 20;  // rows of a bin buffer to begin with
+  Slot& B = E->slots[0];
   if (!E->d_lin) {
     if ((e = dmalloc(&E->d_lin, pq::LIN_WORDS * 4)) != cudaSuccess) return E->cuda_fail(e, "hash tables");
     cudaMemcpyAsync(E->d_lin, lin_table().data(), pq::LIN_WORDS * 4, cudaMemcpyHostToDevice, E->stream);
   }
-  if (!S.counts && (e = dmalloc(&S.counts, 3 * (size_t)pq::COUNT_WORDS * 4)) != cudaSuccess)
+  if (!B.counts && (e = dmalloc(&B.counts, 3 * (size_t)pq::COUNT_WORDS * 4)) != cudaSuccess)
     return E->cuda_fail(e, "bin counters");
   const size_t nw = std::max<size_t>(P.windows.size(), 1);
   if (S.windows_cap < nw) {  // windows, and the state with the growth table behind it
@@ -1518,7 +1521,7 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
       cudaSuccess)
     return E->cuda_fail(e, "windows");
   for (int i = 0; i < 2; ++i)
-    if (int rc = E->ensure_bins(S, i, std::max(ROOM, S.bin_W[i] == W ? S.room[i] : 0), W)) return rc;
+    if (int rc = E->ensure_bins(B, i, ROOM, W)) return rc;
   upload_ops(E, S, P);
   if (no) {
     cudaMemcpyAsync(S.d_windows, P.windows.data(), P.windows.size() * sizeof(pq::WinDesc), cudaMemcpyHostToDevice,
@@ -1529,7 +1532,6 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     cudaMemsetAsync(S.tickets, 0, no * 4, E->stream);
     cudaMemsetAsync(S.stamps, 0, no * 8, E->stream);
   }
-  cudaMemsetAsync(S.counts, 0, 3 * (size_t)pq::COUNT_WORDS * 4, E->stream);
   cudaMemsetAsync(S.bin_state, 0, sizeof(pq::BinState) + 3 * nw * sizeof(float), E->stream);
   pq::BinArgs a{};
   a.ops = S.d_ops;
@@ -1548,33 +1550,70 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
   a.has_min_coeff = P.has_c;
   a.min_coeff = P.ccut;
   a.n0 = P.n0;
-  a.counts = S.counts;
   a.count_words = pq::COUNT_WORDS;
   a.growth = S.growth;
   a.born = S.tickets;
   a.anti = S.anti;
   a.hist = S.hist;
   a.stamps = S.stamps;
-  a.st = E->d_states;
+  a.st = st;
   a.bs = S.bin_state;
   a.hold_block = E->lim.hold_block;
   a.hold_us = std::min<u32>(E->lim.hold_us, 100000);
-  const int grid = with_bins(W, P.alg, [](auto w, auto alg) { return pq::bins_grid<w, alg>(); });
-  if (grid <= 0) return E->fail(PQ_ERR_CUDA, "the binned sweep does not fit this device");
+  *out = a;
+  return PQ_OK;
+}
+
+// The buffers a launch runs on (they move when they grow), and their counters
+// cleared for a sweep from the start.
+void bind_bins(pq_engine* E, Slot& S, pq::BinArgs& a) {
+  const Slot& B = E->slots[0];
+  for (int i = 0; i < 2; ++i) {
+    a.bin_keys[i] = B.bin_keys[i];
+    a.bin_coeffs[i] = B.bin_coeffs[i];
+    a.bin_hash[i] = B.bin_hash[i];
+    a.spill_bin[i] = B.spill_bin[i];
+    a.room[i] = B.room[i];
+  }
+  a.counts = B.counts;
+  a.keys = S.keys[S.cur];
+  a.coeffs = S.coeffs[S.cur];
+  a.dense_room = S.cap;
+}
+void clear_counts(pq_engine* E) {
+  cudaMemsetAsync(E->slots[0].counts, 0, 3 * (size_t)pq::COUNT_WORDS * 4, E->stream);
+}
+
+int bins_error(pq_engine* E, const pq::SweepState& h) {
+  if (h.error & pq::ERR_BARRIER_TIMEOUT)
+    return E->fail(PQ_ERR_DEVICE_TIMEOUT, "a grid barrier wait expired on the device");
+  if (h.error) return E->fail(PQ_ERR_CUDA, "device reported error bits " + std::to_string(h.error));
+  return PQ_OK;
+}
+
+int bins_grid_for(pq_engine* E, const Plan& P, int* grid) {
+  *grid = with_bins(P.W, P.alg, [](auto w, auto alg) { return pq::bins_grid<w, alg>(); });
+  return *grid > 0 ? PQ_OK : E->fail(PQ_ERR_CUDA, "the binned sweep does not fit this device");
+}
+
+// Runs every op of a plan on the binned sweep: one block alone while the rows
+// fit it, then the windows on the whole grid; a buffer that turned out too
+// small is grown and the sweep goes on from the window that needed it.
+int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
+  cudaError_t e;
+  const int W = P.W;
+  const size_t no = P.ops.size();
+  Slot& B = E->slots[0];
+  pq::BinArgs a{};
+  int grid = 0;
+  if (int rc = bins_grid_for(E, P, &grid)) return rc;
+  if (int rc = prepare_bins(E, S, P, E->d_states, &a)) return rc;
+  clear_counts(E);
   if (!E->h_bins && (e = cudaMallocHost(&E->h_bins, sizeof(pq::BinState))) != cudaSuccess)
     return E->cuda_fail(e, "bin state");
   pq::BinState& hb = *E->h_bins;
   for (bool first = true;; first = false) {
-    for (int i = 0; i < 2; ++i) {
-      a.bin_keys[i] = S.bin_keys[i];
-      a.bin_coeffs[i] = S.bin_coeffs[i];
-      a.bin_hash[i] = S.bin_hash[i];
-      a.spill_bin[i] = S.spill_bin[i];
-      a.room[i] = S.room[i];
-    }
-    a.keys = S.keys[S.cur];
-    a.coeffs = S.coeffs[S.cur];
-    a.dense_room = S.cap;
+    bind_bins(E, S, a);
     if (first) {
       E->h_states[0] = fresh_state(E, P);
       cudaMemcpyAsync(E->d_states, E->h_states, sizeof(pq::SweepState), cudaMemcpyHostToDevice, E->stream);
@@ -1602,9 +1641,7 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     cudaEventElapsedTime(&ms, E->ev_l0, E->ev_l1);
     P.sweep_ms += ms;
     const pq::SweepState& h = E->h_states[0];
-    if (h.error & pq::ERR_BARRIER_TIMEOUT)
-      return E->fail(PQ_ERR_DEVICE_TIMEOUT, "a grid barrier wait expired on the device");
-    if (h.error) return E->fail(PQ_ERR_CUDA, "device reported error bits " + std::to_string(h.error));
+    if (int rc = bins_error(E, h)) return rc;
     if (!hb.stopped) {
       P.n_live = h.n[0];
       P.done = no;
@@ -1615,13 +1652,13 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     if (!hb.dense_start && P.windows.back().op_end > hb.op && P.windows.back().op <= hb.op) {
       if (int rc = E->ensure_dense(S, next_pow2(std::max<u64>(hb.n_dense, S.cap + 1)), 0, W)) return rc;
     } else {
-      const u64 want = std::max<u64>(4 * S.room[fill & 1], next_pow2(4 * hb.rows));
-      if (int rc = E->ensure_bins(S, (int)(fill & 1), want, W)) return rc;
+      const u64 want = std::max<u64>(4 * B.room[fill & 1], next_pow2(4 * hb.rows));
+      if (int rc = E->ensure_bins(B, (int)(fill & 1), want, W)) return rc;
     }
     // Everything the stopped window counted is dropped.
     for (u32 s = 0; s < 3; ++s) {
       if (!hb.dense_start && s == hb.phase % 3) continue;
-      cudaMemsetAsync(S.counts + (size_t)s * pq::COUNT_WORDS, 0, (size_t)pq::COUNT_WORDS * 4, E->stream);
+      cudaMemsetAsync(B.counts + (size_t)s * pq::COUNT_WORDS, 0, (size_t)pq::COUNT_WORDS * 4, E->stream);
       hb.n_spill[s] = 0;
     }
     for (u32 s = 0; s < 3; ++s) {
@@ -2338,6 +2375,113 @@ std::vector<u32> share_blocks(const std::vector<Plan>& plans, const std::vector<
   return cnt;
 }
 
+// Expectation values and results of a batch whose sweeps have run.  sweep_ms
+// below 0: the whole device time.
+int finish_batch(pq_engine* E, const std::vector<Inputs>& ins, std::vector<Plan>& plans, bool began, double sweep_ms) {
+  const size_t n = ins.size();
+  cudaError_t e;
+  if (!began) cudaEventRecord(E->ev_begin, E->stream);
+  std::vector<std::vector<pq::ExpectPartial>> parts(n);
+  for (size_t i = 0; i < n; ++i)
+    if (int rc = finalize(E, E->slots[i], plans[i], &parts[i])) return rc;
+  cudaEventRecord(E->ev_end, E->stream);
+  if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "finalize");
+  float ms = 0;
+  cudaEventElapsedTime(&ms, E->ev_begin, E->ev_end);
+  for (size_t i = 0; i < n; ++i) {
+    if (int rc = finish(E, E->slots[i], plans[i], parts[i])) return rc;
+    ins[i].res->device_ms = ms;  // the batch's device time
+    ins[i].res->sweep_ms = sweep_ms < 0 ? ms : sweep_ms;
+  }
+  return PQ_OK;
+}
+
+// A batch on the binned sweep, one instance after another on the whole grid,
+// except that the solo runs of all of them go side by side first, a block
+// each: sweeps of small instances end there.  An instance whose buffers turn
+// out too small is run again by itself, which grows them.
+int run_batch_bins(pq_engine* E, std::vector<Plan>& plans) {
+  const size_t n = plans.size();
+  cudaError_t e;
+  std::vector<pq::BinArgs> args(n);
+  std::vector<std::pair<int, u32>> order;  // by width
+  std::vector<int> grid(n);
+  for (size_t i = 0; i < n; ++i) {
+    if (int rc = bins_grid_for(E, plans[i], &grid[i])) return rc;
+    if (int rc = prepare_bins(E, E->slots[i], plans[i], E->d_states + i, &args[i])) return rc;
+    E->h_states[i] = fresh_state(E, plans[i]);
+    order.push_back({plans[i].W, (u32)i});
+  }
+  std::stable_sort(order.begin(), order.end());
+  // the solo launches read their arguments from memory, in launch order
+  if ((e = E->batch_args.ensure(n * sizeof(pq::BinArgs))) != cudaSuccess) return E->cuda_fail(e, "batch arguments");
+  std::vector<pq::BinArgs> by_width(n);
+  for (size_t k = 0; k < n; ++k) {
+    const u32 i = order[k].second;
+    for (int b = 0; b < 2; ++b)  // room at this instance's width
+      if (int rc = E->ensure_bins(E->slots[0], b, 0, plans[i].W)) return rc;
+    bind_bins(E, E->slots[i], args[i]);
+    by_width[k] = args[i];
+  }
+  pq::BinArgs* d_args = E->batch_args.at<pq::BinArgs>(0);
+  cudaMemcpyAsync(E->d_states, E->h_states, n * sizeof(pq::SweepState), cudaMemcpyHostToDevice, E->stream);
+  cudaMemcpyAsync(d_args, by_width.data(), n * sizeof(pq::BinArgs), cudaMemcpyHostToDevice, E->stream);
+  cudaEventRecord(E->ev_begin, E->stream);
+  for (size_t k = 0; k < n;) {
+    size_t m = k;
+    while (m < n && order[m].first == order[k].first) ++m;
+    ++E->launches;
+    e = with_bins(order[k].first, plans[0].alg, [&](auto w, auto alg) {
+      return pq::launch_solo_batch<w, alg>(d_args + k, (int)(m - k), E->stream);
+    });
+    if (e != cudaSuccess) return E->cuda_fail(e, "solo launch");
+    k = m;
+  }
+  cudaMemcpyAsync(E->h_states, E->d_states, n * sizeof(pq::SweepState), cudaMemcpyDeviceToHost, E->stream);
+  if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "solo runs");
+  std::vector<u32> rest;
+  for (size_t i = 0; i < n; ++i) {
+    plans[i].sweep_launches = 1;
+    if (int rc = bins_error(E, E->h_states[i])) return rc;
+    if (E->h_states[i].end_op < plans[i].ops.size()) rest.push_back((u32)i);
+  }
+  for (u32 i : rest) {
+    clear_counts(E);
+    ++E->launches;
+    ++plans[i].sweep_launches;
+    e = with_bins(plans[i].W, plans[i].alg,
+                  [&](auto w, auto alg) { return pq::launch_bins<w, alg>(args[i], grid[i], E->stream); });
+    if (e != cudaSuccess) return E->cuda_fail(e, "binned sweep launch");
+  }
+  std::vector<pq::BinState> hb(n);
+  if (!rest.empty()) {
+    cudaMemcpyAsync(E->h_states, E->d_states, n * sizeof(pq::SweepState), cudaMemcpyDeviceToHost, E->stream);
+    for (u32 i : rest)
+      cudaMemcpyAsync(&hb[i], E->slots[i].bin_state, sizeof(pq::BinState), cudaMemcpyDeviceToHost, E->stream);
+    if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "binned sweep");
+  }
+  for (size_t i = 0; i < n; ++i) {
+    Plan& P = plans[i];
+    if (int rc = bins_error(E, E->h_states[i])) return rc;
+    P.n_live = E->h_states[i].n[0];
+    P.done = P.ops.size();
+  }
+  for (u32 i : rest) {
+    if (!hb[i].stopped) continue;
+    Plan& P = plans[i];
+    const u64 launches = P.sweep_launches;
+    P.n0 = P.hc.size();
+    P.uploaded_ops = P.uploaded_gdesc = 0;
+    P.n_live = P.peak = P.n0;
+    P.done = 0;
+    if (int rc = setup_slot(E, E->slots[i], P)) return rc;
+    bool began = true;
+    if (int rc = execute_bins(E, E->slots[i], P, &began)) return rc;
+    P.sweep_launches += launches;
+  }
+  return PQ_OK;
+}
+
 // A batch in cooperative launches of batch_sweep_kernel: every unfinished
 // instance gets a contiguous slice of the grid (at least one block) and runs
 // its own op sequence with its own barrier.  When rebalance_pct of the grid
@@ -2345,7 +2489,7 @@ std::vector<u32> share_blocks(const std::vector<Plan>& plans, const std::vector<
 // rest stop at their next op boundary and the next launch re-splits the whole
 // grid among the instances still running; instances that halted for capacity
 // are grown first.
-int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_batch_tuning& tune) {
+int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_batch_tuning& tune, bool bins = true) {
   const size_t n = ins.size();
   const int alg = (int)ins[0].cfg->basis_kind;
   if (int rc = E->ensure_slots(n)) return rc;
@@ -2355,9 +2499,24 @@ int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_bat
                    "a batch cannot decide Clifford deferral under a TermBudget floor with a weight cut; run that "
                    "instance with pq_run");
   };
+  // The binned sweep runs the instances at their own widths; a batch that
+  // sets parameters of the shared row sweep, or holds an instance the binned
+  // one does not run, takes the row sweep.
+  bool binned = bins && !tune.blocks_per_sm && !tune.fuse_max && !tune.tile_items && !tune.bucket_slots;
+  for (size_t i = 0; i < n && binned; ++i) {
+    Plan probe;
+    probe.in = &ins[i];
+    probe.W = ins[i].in_words;
+    probe.has_floor = ins[i].cfg->min_terms >= 0;
+    probe.log = ins[i].cfg->log_gates != 0;
+    const Plugin* np = reinterpret_cast<const Plugin*>(ins[i].cfg->noise_plugin);
+    probe.host_ops = ins[i].cfg->truncator || (ins[i].cfg->noise_kind == PQ_NOISE_PLUGIN && np && (np->depends & 1));
+    binned = use_bins(E, probe);
+  }
   for (size_t i = 0; i < n; ++i) {
-    const int W = std::max(ins[i].in_words, WM > 1 ? WM / 2 : 1);
+    const int W = binned ? ins[i].in_words : std::max(ins[i].in_words, WM > 1 ? WM / 2 : 1);
     if (int rc = prepare(E, plans[i], ins[i], W)) return rc;
+    plans[i].binned = binned;
     if (plans[i].host_ops)
       return E->fail(PQ_ERR_UNSUPPORTED, "a batch does not run truncator plugins or key-reading noise; use pq_run");
     if (tune.fuse_max) plans[i].fuse_max = tune.fuse_max;
@@ -2365,9 +2524,24 @@ int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_bat
     if (tune.bucket_slots) plans[i].bucket_slots = tune.bucket_slots;
     if (int rc = setup_slot(E, E->slots[i], plans[i])) return rc;
     if (int rc = build_ops(plans[i], no_sync)) return rc;
+    if (binned) {
+      plan_windows(plans[i]);
+      continue;
+    }
     fuse_classes(plans[i]);
     fuse_groups(plans[i]);
     upload_ops(E, E->slots[i], plans[i]);
+  }
+  if (binned) {
+    const int rc = run_batch_bins(E, plans);
+    if (rc == PQ_ERR_OOM) {  // the row sweep may still fit
+      E->slots[0].free_bins(0);
+      E->slots[0].free_bins(1);
+      for (size_t i = 0; i < n; ++i) E->slots[i].free_rows();
+      return run_batch(E, ins, WM, tune, false);
+    }
+    if (rc) return rc;
+    return finish_batch(E, ins, plans, true, -1.0);
   }
   const int grid_max = with_words(WM, [&](auto w) {
     constexpr int WW = decltype(w)::value;
@@ -2429,20 +2603,7 @@ int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_bat
     for (size_t k = 0; k < todo.size(); ++k)
       if (int rc = absorb_state(E, E->slots[todo[k]], plans[todo[k]], E->h_states[k])) return rc;
   }
-  if (!began) cudaEventRecord(E->ev_begin, E->stream);
-  std::vector<std::vector<pq::ExpectPartial>> parts(n);
-  for (size_t i = 0; i < n; ++i)
-    if (int rc = finalize(E, E->slots[i], plans[i], &parts[i])) return rc;
-  cudaEventRecord(E->ev_end, E->stream);
-  if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "finalize");
-  float ms = 0;
-  cudaEventElapsedTime(&ms, E->ev_begin, E->ev_end);
-  for (size_t i = 0; i < n; ++i) {
-    if (int rc = finish(E, E->slots[i], plans[i], parts[i])) return rc;
-    ins[i].res->device_ms = ms;  // the batch's device time
-    ins[i].res->sweep_ms = sweep_ms;
-  }
-  return PQ_OK;
+  return finish_batch(E, ins, plans, began, sweep_ms);
 }
 
 }  // namespace

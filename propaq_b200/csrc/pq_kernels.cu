@@ -1405,6 +1405,15 @@ __global__ void __launch_bounds__(BinSize<W>::T, 1) solo_kernel(const __grid_con
   solo_body<W, ALG>(a, s.warp, s.block);
 }
 template <int W, int ALG>
+__global__ void __launch_bounds__(BinSize<W>::T, 1) solo_batch_kernel(const BinArgs* args) {
+  extern __shared__ __align__(16) unsigned char bin_smem[];
+  __shared__ BinArgs sa;
+  if (threadIdx.x == 0) sa = args[blockIdx.x];
+  __syncthreads();
+  auto& s = *reinterpret_cast<typename BinSize<W>::SoloSmem*>(bin_smem);
+  solo_body<W, ALG>(sa, s.warp, s.block);
+}
+template <int W, int ALG>
 __global__ void __launch_bounds__(BinSize<W>::T, BinSize<W>::BLOCKS) bins_kernel(const __grid_constant__ BinArgs a) {
   extern __shared__ __align__(16) unsigned char bin_smem[];
   auto& s = *reinterpret_cast<typename BinSize<W>::GridSmem*>(bin_smem);
@@ -1824,6 +1833,16 @@ cudaError_t launch_solo(const BinArgs& a, cudaStream_t s) {
 }
 
 template <int W, int ALG>
+cudaError_t launch_solo_batch(const BinArgs* args, int n, cudaStream_t s) {
+  using S = typename BinSize<W>::SoloSmem;
+  if (cudaError_t e = cudaFuncSetAttribute(solo_batch_kernel<W, ALG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(S)))
+    return e;
+  solo_batch_kernel<W, ALG><<<n, BinSize<W>::T, sizeof(S), s>>>(args);
+  return cudaGetLastError();
+}
+
+template <int W, int ALG>
 int bins_grid() {
   using S = typename BinSize<W>::GridSmem;
   static_assert(BinSize<W>::BLOCKS * (sizeof(S) + 1024) <= 228 * 1024, "resident blocks");
@@ -1928,6 +1947,7 @@ cudaError_t launch_conjugate(const u64* keys, const double* coeffs, u64 n, const
 #define PQ_INSTANTIATE_BINS(Wv, Av)                                                                     \
   template int bins_grid<Wv, Av>();                                                                     \
   template cudaError_t launch_solo<Wv, Av>(const BinArgs&, cudaStream_t);                               \
+  template cudaError_t launch_solo_batch<Wv, Av>(const BinArgs*, int, cudaStream_t);                     \
   template cudaError_t launch_bins<Wv, Av>(const BinArgs&, int, cudaStream_t);
 #define PQ_INSTANTIATE_KEYS(Wv)                                                                         \
   template cudaError_t launch_rebuild<Wv>(const u64*, u64, u64*, u64, u64, u32*, cudaStream_t);         \

@@ -238,6 +238,9 @@ int bins_grid();
 // where it stopped (st->end_op) on the whole grid.
 template <int W, int ALG>
 cudaError_t launch_solo(const BinArgs& a, cudaStream_t s);
+// The solo runs of n propagations, a block each (args on the device).
+template <int W, int ALG>
+cudaError_t launch_solo_batch(const BinArgs* args, int n, cudaStream_t s);
 template <int W, int ALG>
 cudaError_t launch_bins(const BinArgs& a, int grid, cudaStream_t s);
 

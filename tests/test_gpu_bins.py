@@ -9,6 +9,7 @@ coefficient bit for bit, terms below the cutoff, expectation value.
 * groups as large as a window's span allows (dense cosets), and more rows than
   the bins hold, so that bins are split;
 * buffers that grow mid-run on a fresh engine, final rows included;
+* the same in a batch, whose instances share those buffers;
 * weight cuts around the limit of disjoint windows, phase-only rotations,
   layered noise tables, empty layers, odd Majorana generators."""
 
@@ -17,7 +18,7 @@ import math
 import numpy as np
 import pytest
 from harness import (Problem, assert_terms_equal, expectation_close, from_circuit, from_workload,
-                     random_pauli_problem, run_gpu, run_oracle)
+                     random_pauli_problem, run_gpu, run_gpu_batch, run_oracle)
 
 from propaq_b200 import _native, workloads
 from propaq_b200.circuits import MajoranaCircuit, MajoranaRotation, PauliCircuit, PauliRotation
@@ -81,6 +82,25 @@ def test_buffers_grow_on_a_fresh_engine(oracle, make):
     b = run_gpu(engine, p)  # nothing left to grow
     assert a.res.sweep_launches >= b.res.sweep_launches
     assert np.array_equal(a.keys, b.keys) and np.array_equal(a.coeffs, b.coeffs) and a.expectation == b.expectation
+
+
+def test_batch_grows_on_a_fresh_engine(oracle):
+    # Instances of every width, some ending solo, two outgrowing their buffers
+    # (they are run again by themselves), one observable folded on the device.
+    engine = _native.Engine(0)
+    probs = [from_workload(w) for w in (workloads.kicked_ising(4, 4, 6), workloads.tfim_chain(8, 2),
+                                        workloads.kicked_ising(6, 6, 6), workloads.kicked_ising(9, 15, 3),
+                                        workloads.kicked_ising(7, 10, 2), workloads.tfim_chain(20, 6))]
+    base = random_pauli_problem(3, 20, n_gates=24, max_weight=6, min_coeff=1e-3)
+    keys, coeffs = observable(20, 12000, 1, 3)
+    probs.append(Problem(0, 20, 1, np.concatenate([keys] * 3), np.concatenate([coeffs, 0.5 * coeffs, coeffs]),
+                         base.gate_keys, base.angles, base.offsets, base.diag, 6, 1e-3))
+    for _ in range(2):
+        for p, b in zip(probs, run_gpu_batch(engine, probs)):
+            o = run_oracle(oracle, p)
+            assert np.array_equal(b.n_terms, o.n_terms)
+            assert_terms_equal(b.keys, b.coeffs, o.keys, o.coeffs)
+            assert expectation_close(b.expectation, o)[0]
 
 
 @pytest.mark.parametrize("shape,cut", [((5, 7), 10), ((5, 7), 11), ((5, 7), 12), ((9, 15), 10), ((9, 15), 11)])
