@@ -777,8 +777,8 @@ def main():
            + (0 if table is None else table.nbytes))
     d2h = 8 * len(prob.angles) + 16 * n_ops + 32 * 4 * 148
     peak_gbs, peak_kind = measured_peaks()
-    # The dominant kernel is the sweep: one cooperative launch per step (plus
-    # one per capacity growth) runs every gate and noise op.
+    # The dominant kernels are the sweep's: a solo launch and a grid launch per
+    # step (plus one per buffer growth) run every gate and noise op.
     achieved = alg_bytes / (sweep_ms / 1e3) / 1e9 if sweep_ms > 0 else None
     # DRAM bytes of the sweep launches of one step, from an ncu capture
     # (profiles/sweep_traffic_*.json), as bytes per launch like `achieved`:
@@ -803,7 +803,7 @@ def main():
                 gpu_launches=launches,
                 roofline={"bound": "hbm", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s",
                           "frac": None if achieved is None else achieved / peak_gbs, "traffic": traffic,
-                          "kernel": "sweep_kernel", "peak_source": f"{peak_kind} hbm_gbs",
+                          "kernel": "bins_kernel + solo_kernel", "peak_source": f"{peak_kind} hbm_gbs",
                           "launches": sweep_launches,
                           "algorithmic_bytes_per_launch": alg_bytes / max(1, sweep_launches),
                           "ms_per_launch": sweep_ms / max(1, sweep_launches),

@@ -81,8 +81,9 @@ typedef struct pq_run_config {
   size_t noise_table_len;    /* entries per table (normally n_units + 1)       */
   const pq_plugin* noise_plugin; /* PLUGIN kind                                 */
   uint32_t want_terms;       /* keep the final terms for pq_result_terms: 1 in
-                                the engine's row order, 2 sorted by key (as a
-                                64 n_words-bit integer, on the device)          */
+                                an order of the engine's, the same in every
+                                run; 2 sorted by key (as a 64 n_words-bit
+                                integer, on the device)                         */
   uint32_t blocks_per_sm;    /* sweep blocks per SM; 0 = by live count: 1 while
                                 every row has a thread, 2 up to 2^20 rows, then
                                 as many as fit (a launch stops and is relaunched
@@ -96,7 +97,9 @@ typedef struct pq_run_config {
   uint32_t tile_items;       /* rows per thread of a many-row gate tile: 1-4
                                 (default 4)                                     */
   uint32_t bucket_slots;     /* hash-table slots a key's probe starts in: 2, 4
-                                or 8 (default 2)                                */
+                                or 8 (default 2).  These three and blocks_per_sm
+                                are parameters of the row sweep: a run that sets
+                                one takes it instead of the binned sweep        */
 } pq_run_config;
 
 /* crates/core/src/interface/results.rs:8-51 (PropagationResult), plus the
@@ -122,8 +125,8 @@ typedef struct pq_result {
   uint64_t sum_rows_phase;    /* sum over phase-only ops of the rows they scan */
   uint64_t sum_rows_noise;    /* sum over noise ops of the rows they scan      */
   uint64_t sum_kept;          /* ... of the rows a reclaim keeps               */
-  uint64_t class_ops;         /* ops that ran a class of rotations (generators on
-                                 disjoint units) through one pass              */
+  uint64_t class_ops;         /* runs of four or more Clifford rotations on
+                                 disjoint units that went through one pass     */
 } pq_result;
 
 /* Key width for a register: 1,2,4,...,64 words for up to 32,64,...,2048
@@ -246,10 +249,13 @@ typedef struct pq_batch_tuning {
   uint32_t bucket_slots;
 } pq_batch_tuning;
 
-/* Runs n independent propagations of one basis in shared persistent
- * launches: each instance owns a slice of the co-resident grid and runs its
- * op sequence there with its own grid barrier, so small instances fill the
- * GPU together and no instance pays a launch per gate.  The reference runs
+/* Runs n independent propagations of one basis in one call: the starts of
+ * all of them side by side, a block each, then those that outgrow a block one
+ * after another on the whole grid.  A batch that sets blocks_per_sm or a
+ * kernel knob, or holds an instance the binned sweep does not run, shares
+ * persistent launches instead: each instance owns a slice of the co-resident
+ * grid and runs its op sequence there with its own grid barrier (split and
+ * rebalance_pct act there).  The reference runs
  * such sweeps as one expectation_value call after another
  * (ZeroNoiseExtrapolator.run / ZeroCutoffExtrapolator.run,
  * propaq/extrapolators/zne.py:63-108, zce.py:88-137); each instance gives

@@ -1,7 +1,12 @@
 // pq_kernels.cu -- the hot path of the B200 propagation engine.
 //
-// The whole op sequence of a propagation (noise layers and gates, in
-// Heisenberg order) runs as ONE cooperative persistent kernel, sweep_kernel.
+// Most propagations run on the binned sweep (pq_bins.cuh, solo_kernel and
+// bins_kernel below).  The rest -- a TermBudget floor, plugins asked per row,
+// the verbose log, the gradient's recorded forward pass, wide keys -- run on
+// the row sweep, which this file describes first.
+//
+// The row sweep: the whole op sequence of a propagation (noise layers and
+// gates, in Heisenberg order) as ONE cooperative persistent kernel, sweep_kernel.
 // Its blocks are co-resident; a bounded grid barrier separates consecutive
 // ops, so a gate costs no launch.  Per gate the kernel replaces the
 // reference's scan -> route -> absorb -> claim -> rescue rounds

@@ -265,8 +265,8 @@ class _Propagator:
 
 def expectation_values(jobs, blocks_per_sm: int = 0, split: int = 1, rebalance_pct: int = 25, device: int = 0,
                        autotune: bool = False, fuse_max: int = 0, tile_items: int = 0, bucket_slots: int = 0):
-    """Expectation values of many independent propagations in shared
-    persistent launches on one GPU (pq_run_batch).
+    """Expectation values of many independent propagations in one call on one
+    GPU (pq_run_batch).
 
     `jobs` is a list of (propagator, observable, circuit, initial_state); all
     propagators are Pauli or all Majorana, each with its own noise and
@@ -278,7 +278,7 @@ def expectation_values(jobs, blocks_per_sm: int = 0, split: int = 1, rebalance_p
     blocks_per_sm: grid size per SM (0 = as many as fit); split: 0 shares the
     grid equally among the jobs, 1 in proportion to their remaining work;
     rebalance_pct: re-split the grid among the running jobs once this share of
-    it is idle (0 = never).  fuse_max, tile_items, bucket_slots: the kernel
+    it is idle (0 = never); both act on batches the row sweep runs.  fuse_max, tile_items, bucket_slots: the kernel
     knobs of pq_batch_tuning (0 = the engine's defaults).  autotune: choose all
     six by measurement instead (propaq_b200.tuning; the first batch of a shape
     runs once per setting tried, later ones reuse the choice).
