@@ -1,0 +1,86 @@
+"""Windows of the binned sweep (propaq_b200/csrc/pq_host.cu, plan_windows)
+against the oracle: live count after every rotation, branching rows, term set,
+every coefficient bit for bit, expectation value.
+
+* Rotations by pi across a layer of rotations on disjoint qubits: they share
+  its window and need not commute with it, so a row born inside the window may
+  anticommute with one although no row entering it does."""
+
+from __future__ import annotations
+
+import math
+
+import numpy as np
+import pytest
+from harness import (assert_terms_equal, expectation_close, from_circuit, run_gpu, run_gpu_batch, run_oracle)
+
+from propaq_b200.circuits import PauliCircuit, PauliRotation
+from propaq_b200.datatypes import PauliString, PauliTermSum
+
+
+def check(g, o):
+    assert np.array_equal(g.n_terms, o.n_terms), "live counts per gate differ"
+    assert_terms_equal(g.keys, g.coeffs, o.keys, o.coeffs)
+    assert g.terms_below_cutoff == o.terms_below_cutoff
+    assert expectation_close(g.expectation, o)[0]
+
+
+def echo(n, cut):
+    """Z on qubit 0 under RX(0.3), RZ(pi), RX(0.3) on every qubit: the second
+    layer undoes the first, <Z> = 1."""
+    x = [PauliRotation(PauliString(1 << q, 0, n), 0.3) for q in range(n)]
+    z = [PauliRotation(PauliString(0, 1 << q, n), math.pi) for q in range(n)]
+    return from_circuit(0, n, PauliTermSum({PauliString(0, 1, n): 1.0}), PauliCircuit([x, z, x]), 0, max_weight=cut)
+
+
+def pulses(seed, n, n_terms, cut, min_coeff):
+    """Layers of one-qubit rotations on every qubit, with rotations by multiples
+    of pi about random one- and two-qubit Paulis between and after them."""
+    rng = np.random.default_rng(seed)
+
+    def pauli(k):
+        x = z = 0
+        for q in rng.choice(n, size=k, replace=False):
+            t = int(rng.integers(1, 4))
+            x |= (t & 1) << int(q)
+            z |= (t >> 1) << int(q)
+        return PauliString(x, z, n)
+
+    layers = []
+    for _ in range(3):
+        layer = []
+        for q in range(n):
+            t = int(rng.integers(1, 4))
+            layer.append(PauliRotation(PauliString((t & 1) << q, (t >> 1) << q, n), float(rng.uniform(0.1, 1.4))))
+            if rng.random() < 0.3:
+                layer.append(PauliRotation(pauli(int(rng.integers(1, 3))), math.pi * int(rng.integers(1, 4))))
+        layers.append(layer[:126])
+    obs = {}
+    while len(obs) < n_terms:
+        obs[pauli(int(rng.integers(1, 5)))] = float(rng.normal())
+    return from_circuit(0, n, PauliTermSum(obs), PauliCircuit(layers), 5, max_weight=cut, min_coeff=min_coeff)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,cut", [(20, 8), (20, 11), (50, 11), (100, 11), (100, 8), (180, 10)])
+def test_echo_across_a_disjoint_window(gpu_engine, oracle, n, cut):
+    p = echo(n, cut)
+    g = run_gpu(gpu_engine, p)
+    check(g, run_oracle(oracle, p))
+    assert abs(g.expectation - 1.0) < 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,cut", [(20, 11), (50, 10), (100, 11), (180, 10)])
+@pytest.mark.parametrize("n_terms", [1, 40, 500])
+def test_pulses_in_disjoint_windows(gpu_engine, oracle, n, cut, n_terms):
+    # one term: a warp alone; 40: a block; 500: bins of warps and of blocks
+    p = pulses(n + n_terms, n, n_terms, cut, 1e-3)
+    check(run_gpu(gpu_engine, p), run_oracle(oracle, p))
+
+
+@pytest.mark.gpu
+def test_pulses_in_a_batch(gpu_engine, oracle):
+    probs = [echo(20, 9), pulses(1, 30, 4, 10, 1e-3), pulses(2, 60, 60, 9, 1e-2), echo(100, 11)]
+    for p, g in zip(probs, run_gpu_batch(gpu_engine, probs)):
+        check(g, run_oracle(oracle, p))
