@@ -27,7 +27,7 @@ LIB = LIB_DIR / "libpropaq_cuda.so"
 WIDTH_UNITS = ["pq_kernels_w64.cu", "pq_kernels_w64_majorana.cu", "pq_kernels_w32.cu", "pq_kernels_w32_majorana.cu",
                "pq_kernels_w16.cu", "pq_kernels_w4.cu", "pq_kernels_w8.cu"]
 SOURCES = WIDTH_UNITS[:4] + ["pq_kernels.cu"] + WIDTH_UNITS[4:] + ["pq_host.cu", "pq_noalloc.cu", "pq_sort.cu"]
-HEADERS = ["pq_device.cuh", "pq_kernels.cuh", "pq_tableau.h", "pq_class.cuh", "pq_bins.cuh", "pq_sort.cuh"]
+HEADERS = ["pq_device.cuh", "pq_layout.cuh", "pq_kernels.cuh", "pq_tableau.h", "pq_class.cuh", "pq_bins.cuh", "pq_sort.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -61,11 +61,11 @@ def _obj(src: str) -> Path:
 
 
 # What each translation unit includes (besides itself).
-_KERNEL_DEPS = ["pq_device.cuh", "pq_kernels.cuh", "pq_class.cuh", "pq_bins.cuh"]
+_KERNEL_DEPS = ["pq_device.cuh", "pq_layout.cuh", "pq_kernels.cuh", "pq_class.cuh", "pq_bins.cuh"]
 DEPS = {
     "pq_kernels.cu": _KERNEL_DEPS,
     **{u: _KERNEL_DEPS + ["pq_kernels.cu"] for u in WIDTH_UNITS},
-    "pq_host.cu": ["pq_device.cuh", "pq_kernels.cuh", "pq_sort.cuh", "pq_tableau.h", "../../include/propaq_cuda.h"],
+    "pq_host.cu": ["pq_device.cuh", "pq_layout.cuh", "pq_kernels.cuh", "pq_sort.cuh", "pq_tableau.h", "../../include/propaq_cuda.h"],
     "pq_noalloc.cu": ["pq_device.cuh", "../../include/propaq_cuda.h"],
     "pq_sort.cu": ["pq_device.cuh", "pq_sort.cuh"],
 }

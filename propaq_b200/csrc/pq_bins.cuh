@@ -581,40 +581,7 @@ __device__ __forceinline__ void solo_body(const BinArgs& a, SW& sw, SB& sb) {
 }
 
 // ------------------------------------------------------------ binned windows
-// The bins the rows are dealt into: bin b holds rows [b * cap, b * cap +
-// count[b]) of its buffer, and rows past a full bin go to the buffer's spill
-// area, tagged with their bin.
-constexpr u64 SPILL_SHARE = 16;  // of a buffer; more spills than that and the host grows it
-struct Layout {
-  u32 bins, stride;  // counters are `stride` words apart (few bins: a sector or line each)
-  u32 cap;
-};
-
-// Bins for about n rows that a window lets grow by a factor `grow`, grown bins
-// `fill` full.  While a bin of every warp holds at most WARP_ROWS rows when
-// grown, that many (a warp alone runs 32 branching rows at a time, a block
-// 256: bins that grew to 62 rows a warp ran a window of 50 rotations in 79 us
-// (kicked Ising 10x10) against 72 us by blocks, bins of 22 one of 40 in 43
-// against 51 us; where one family fills a bin, as in a TFIM chain's RX layer,
-// the line is lower); else bins of blocks, one each or, up to four, a whole
-// number each (340 bins on 296 blocks cost two rounds).  All the room there
-// is, less the spill area.
-constexpr float WARP_ROWS = 12.0f;
-__device__ __forceinline__ Layout choose_layout(float n, float grow, float fill, u32 blocks, u32 warps, u32 rows,
-                                                u64 room) {
-  Layout l;
-  u64 b = (u64)(n * grow / (fill * (float)rows)) + 1;
-  if (n * grow <= WARP_ROWS * (float)(blocks * warps)) b = (u64)blocks * warps;
-  else if (b < 4ull * blocks) b = (b + blocks - 1) / blocks * blocks;
-  else if (b == (u64)blocks * warps) ++b;  // that number means bins of warps
-  if (b > BIN_MAX) b = BIN_MAX;
-  l.bins = (u32)b;
-  l.stride = b <= 4096 ? 32u : (b <= 16384 ? 8u : 1u);
-  const u64 c = (room - room / SPILL_SHARE) / b;
-  l.cap = c > 0x7fffffffull ? 0x7fffffffu : (u32)c;
-  return l;
-}
-
+// (the layout of the bins: pq_layout.cuh)
 __device__ __forceinline__ u32 bin_of(u32 g, u32 bins) { return __umulhi(g * 0x9E3779B1u, bins); }
 // The bits a bin is split by when it does not fit.
 __device__ __forceinline__ u32 split_bits(u32 g) { return (g ^ (g >> 15)) * 0x85EBCA6Bu; }
@@ -648,7 +615,7 @@ struct Dest {
   u32* n_spill;    // spilled rows
   u64* n_dense;    // dense (no bins): rows written
   u32* fail;       // set when the buffer is full
-  u64 room;        // rows of the buffer (bins, then spills)
+  u64 room;        // rows that may spill; dense: rows of the buffer
   Layout l;
   u32 dense;
 };
@@ -734,11 +701,11 @@ __device__ __forceinline__ void put_row(const WinSmem<W>& v, const u64* k, doubl
       at = (u64)bin * d.l.cap + pos;
     } else {
       const u32 sp = atomicAdd(d.n_spill, 1u);
-      at = (u64)d.l.bins * d.l.cap + sp;
-      if (at >= d.room) {
+      if (sp >= d.room) {
         *d.fail = 1;
         return;
       }
+      at = (u64)d.l.bins * d.l.cap + sp;
       d.spill_bin[sp] = bin;
     }
     d.h[at] = h;
@@ -1011,7 +978,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     d.h = a.bin_hash[set & 1];
     d.cnt = a.counts + (u64)(set % 3) * a.count_words;
     d.spill_bin = a.spill_bin[set & 1];
-    d.room = a.room[set & 1];
+    d.room = spill_room(l, a.room[set & 1]);
     d.n_spill = &bs->n_spill[set % 3];
     d.n_dense = nullptr;
     d.fail = &bs->fail[set % 3];

@@ -575,7 +575,7 @@ struct pq_engine {
       cudaError_t e;
       if ((e = dmalloc(&S.bin_keys[i], nw * 8)) != cudaSuccess || (e = dmalloc(&S.bin_coeffs[i], nr * 8)) != cudaSuccess ||
           (e = dmalloc(&S.bin_hash[i], nr * 4)) != cudaSuccess ||
-          (e = dmalloc(&S.spill_bin[i], nr / 8 * 4)) != cudaSuccess) {
+          (e = dmalloc(&S.spill_bin[i], pq::spill_tags(nr) * 4)) != cudaSuccess) {
         S.free_bins(i);
         return cuda_fail(e, "allocating bins");
       }

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "pq_device.cuh"
+#include "pq_layout.cuh"
 
 namespace pq {
 
@@ -155,8 +156,6 @@ struct SweepArgs {
 // ------------------------------------------------------------ binned sweep
 // See pq_bins.cuh.
 constexpr u32 WIN_MAX = 128;       // rotations of one window
-constexpr u32 BIN_MAX = 1u << 18;  // bins of one buffer
-constexpr u32 COUNT_WORDS = BIN_MAX;  // words of one counter set (fewer bins, wider stride: choose_layout)
 constexpr u32 LIN_WORDS = 8 * 256;  // linear hash: 8 byte tables
 // Largest rank of a span window / family dimension of a disjoint window: a
 // group of 2^rank rows must fit the rows a block holds.

@@ -4,7 +4,9 @@ every coefficient bit for bit, expectation value.
 
 * Rotations by pi across a layer of rotations on disjoint qubits: they share
   its window and need not commute with it, so a row born inside the window may
-  anticommute with one although no row entering it does."""
+  anticommute with one although no row entering it does.
+* Live sets that double with every rotation, so that buffers of the first size
+  are asked for very many bins."""
 
 from __future__ import annotations
 
@@ -14,6 +16,7 @@ import numpy as np
 import pytest
 from harness import (assert_terms_equal, expectation_close, from_circuit, run_gpu, run_gpu_batch, run_oracle)
 
+from propaq_b200 import _native
 from propaq_b200.circuits import PauliCircuit, PauliRotation
 from propaq_b200.datatypes import PauliString, PauliTermSum
 
@@ -84,3 +87,20 @@ def test_pulses_in_a_batch(gpu_engine, oracle):
     probs = [echo(20, 9), pulses(1, 30, 4, 10, 1e-3), pulses(2, 60, 60, 9, 1e-2), echo(100, 11)]
     for p, g in zip(probs, run_gpu_batch(gpu_engine, probs)):
         check(g, run_oracle(oracle, p))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,width", [(24, 200), (25, 90), (26, 26)], ids=["W8", "W4", "W1"])
+def test_doubling_past_every_buffer(n, width):
+    # Z on n qubits under RX on each of them: 2^n rows, <0|..|0> = prod cos.  A
+    # fresh engine, so every buffer starts at its first size.
+    rng = np.random.default_rng(n)
+    angles = rng.uniform(0.3, 1.2, n)
+    x = [PauliRotation(PauliString(1 << q, 0, width), float(angles[q])) for q in range(n)]
+    zz = [PauliRotation(PauliString(0, 3 << q, width), 0.4) for q in (0, 2)]
+    p = from_circuit(0, width, PauliTermSum({PauliString(0, (1 << n) - 1, width): 1.0}), PauliCircuit([zz, x]), 0)
+    g = run_gpu(_native.Engine(0), p, want_terms=False)
+    # every row has Y or Z on each qubit; of the four pairs a ZZ rotation
+    # branches two, into two new ones
+    assert g.n_terms.tolist() == [2 << q for q in range(n)] + [3 << (n - 1), 9 << (n - 2)]
+    assert abs(g.expectation - float(np.prod(np.cos(angles)))) < 1e-12
