@@ -1587,7 +1587,11 @@ void clear_counts(pq_engine* E) {
   cudaMemsetAsync(E->slots[0].counts, 0, 3 * (size_t)pq::COUNT_WORDS * 4, E->stream);
 }
 
+// Not an error of the caller's: a bin that no further bit of the group hash
+// splits holds more rows than a block does.  The row sweep runs such a call.
+constexpr int BINS_UNFIT = -1000;
 int bins_error(pq_engine* E, const pq::SweepState& h) {
+  if (h.error == pq::ERR_CAPACITY) return E->fail(BINS_UNFIT, "a bin cannot be split");
   if (h.error & pq::ERR_BARRIER_TIMEOUT)
     return E->fail(PQ_ERR_DEVICE_TIMEOUT, "a grid barrier wait expired on the device");
   if (h.error) return E->fail(PQ_ERR_CUDA, "device reported error bits " + std::to_string(h.error));
@@ -2084,8 +2088,8 @@ int run_one(pq_engine* E, const Inputs& in, int W, bool bins = true) {
       S.free_bins(0);
       S.free_bins(1);
       S.free_rows();
-      return run_one(E, in, W, false);
     }
+    if (rc == PQ_ERR_OOM || rc == BINS_UNFIT) return run_one(E, in, W, false);
     if (rc) return rc;
   } else {
     fuse_classes(P);
@@ -2541,8 +2545,8 @@ int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_bat
       E->slots[0].free_bins(0);
       E->slots[0].free_bins(1);
       for (size_t i = 0; i < n; ++i) E->slots[i].free_rows();
-      return run_batch(E, ins, WM, tune, false);
     }
+    if (rc == PQ_ERR_OOM || rc == BINS_UNFIT) return run_batch(E, ins, WM, tune, false);
     if (rc) return rc;
     return finish_batch(E, ins, plans, true, -1.0);
   }

@@ -6,7 +6,9 @@ every coefficient bit for bit, expectation value.
   its window and need not commute with it, so a row born inside the window may
   anticommute with one although no row entering it does.
 * Live sets that double with every rotation, so that buffers of the first size
-  are asked for very many bins."""
+  are asked for very many bins.
+* Groups that the 32-bit group hash cannot tell apart and that one block cannot
+  hold together: the run takes the row sweep."""
 
 from __future__ import annotations
 
@@ -104,3 +106,52 @@ def test_doubling_past_every_buffer(n, width):
     # branches two, into two new ones
     assert g.n_terms.tolist() == [2 << q for q in range(n)] + [3 << (n - 1), 9 << (n - 2)]
     assert abs(g.expectation - float(np.prod(np.cos(angles)))) < 1e-12
+
+
+# ------------------------------------------- groups that cannot be told apart
+def hash_kernel(lowest_bit):
+    """A nonzero one-word key on bits >= lowest_bit whose linear hash (lin_table
+    of pq_host.cu) is 0: keys that differ by it share every group hash."""
+    mask = (1 << 64) - 1
+    x, bits = 0x1234567890ABCDEF, []
+    for _ in range(64):
+        x = (x + 0x9E3779B97F4A7C15) & mask
+        z = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & mask
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+        bits.append(((z ^ (z >> 31)) >> 16) & 0xFFFFFFFF)
+    rows = {}
+    for b in range(lowest_bit, 64):
+        h, c = bits[b], 1 << b
+        while h and h.bit_length() in rows:
+            hh, cc = rows[h.bit_length()]
+            h, c = h ^ hh, c ^ cc
+        if not h:
+            return c
+        rows[h.bit_length()] = (h, c)
+    raise AssertionError("the hash is injective on these bits")
+
+
+def colliding_groups(n):
+    """Two terms whose keys differ by a kernel vector of the hash, each grown
+    to 2^11 rows by RX on qubits 0..10: one unsplittable bin of 4,096 rows."""
+    low = 3  # X and Z bits of qubits 0..10 stay clear of the vector
+    d = hash_kernel(22)
+    z11 = sum(1 << q for q in range(11))
+    dx, dz = (sum(((d >> (2 * q + b)) & 1) << q for q in range(11, 32)) for b in (0, 1))
+    obs = PauliTermSum({PauliString(0, z11, n): 1.0, PauliString(dx, dz | z11, n): 0.5, PauliString(0, low, n): 0.25})
+    rx = [PauliRotation(PauliString(1 << q, 0, n), 0.2 + 0.05 * q) for q in range(11)]
+    rzz = [PauliRotation(PauliString(0, 3 << q, n), 0.3) for q in range(4)]
+    p = from_circuit(0, n, obs, PauliCircuit([rzz, rx]), 0)
+    k0, k1 = (int(k[0]) for k in p.obs_keys[np.argsort(-np.abs(p.obs_coeffs))][:2])
+    assert k0 ^ k1 == d
+    return p
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [32, 120], ids=["W1", "W4"])
+def test_bins_that_cannot_be_split(gpu_engine, oracle, n):
+    p = colliding_groups(n)
+    o = run_oracle(oracle, p)
+    check(run_gpu(gpu_engine, p), o)
+    for g in run_gpu_batch(gpu_engine, [p, p]):
+        check(g, o)
