@@ -747,7 +747,11 @@ __device__ __forceinline__ u32 finish_row(const WinSmem<W>& v, const BinArgs& a,
 // One bin by one unit: its rows into shared memory, the window's rotations,
 // and every row on to its next place.  A block splits what does not fit; a
 // warp returns false instead, having written nothing.  depth0: how deep this
-// block's bins of the window have been split so far.
+// block's bins of the window have been split so far by parts that held no more
+// than their share of the bin.  (Two full groups that agree in many split bits
+// go deep by themselves: counted too, one such pair had the block run all its
+// later bins in 256 parts, 22 rotations that double one row to 2^22 in 4.1 ms
+// instead of 0.9.)
 template <int W, int ALG, class S>
 __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u32 bin, u32& depth0, u32& kept) {
   constexpr int T = S::T;
@@ -794,6 +798,7 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
   // late in a window of 80 rotations takes as long as running it
   while (!WARP && depth < 24 && (float)(n_all >> depth) * v.grow > (float)S::R * 0.9f) ++depth;
   const u32 base = depth;
+  u32 failed = 0;  // rows of the part that failed last: a half that holds them all fails too
   for (;;) {
     for (u32 i = tid; i < G; i += T) {
       s.born[i] = 0;
@@ -836,8 +841,9 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
       unit_sync<S>();
       n = s.n;
     }
-    bool fits = n <= (u32)S::R;
-    if (fits) {
+    const u32 n_load = n;
+    bool fits = n <= (u32)S::R && (!n || n != failed);
+    if (fits && n) {
       const bool some = v.w.commute && n <= ACT_ROWS;
       if (some) {
         unit_sync<S>();
@@ -880,9 +886,11 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
     }
     if (!fits) {
       if (WARP) return false;
+      failed = n_load;
+      const bool fair = n_load <= (n_all >> depth) + (n_all >> (depth + 2));
       ++depth;  // run the part again in halves
+      if (fair && depth0 < depth && depth <= 8) depth0 = depth;
       part <<= 1;
-      if (depth0 < depth && depth0 < 8) depth0 = depth;
       if (depth > 24) {
         if (tid == 0) atomicOr(&a.st->error, ERR_CAPACITY);
         return true;
@@ -890,7 +898,8 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
       unit_sync<S>();
       continue;
     }
-    for (u32 i = tid; i < G; i += T) {
+    if (n) failed = 0;
+    for (u32 i = tid; n && i < G; i += T) {
       if (s.born[i]) atomicAdd(&v.born_all[i], s.born[i]);
       if (s.anti[i]) atomicAdd(&v.anti_all[i], (u32)s.anti[i]);
     }
