@@ -930,6 +930,14 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
   }
 }
 
+// A layout is made before the window that fills it has run.  Rows that came
+// to more than this many times what its bins hold are dealt again first, by
+// their actual number: one pass over the rows, where bins that are split into
+// four parts and more are read as many times.  (From 2^26 rows on in the bins
+// of a few thousand, the two rotations after a doubling window took 3,031 ms
+// of 4-word keys and 64 of 1-word keys; the runs around them now take 31 and 8.)
+constexpr float REDEAL = 2.0f;
+
 // The windows from where the solo run (or a stopped sweep) left off, by the
 // blocks of grp.  SB: a block's rows, SW: a warp's; both lie over one another
 // in `rows`.
@@ -1028,18 +1036,25 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
   }
 
   Layout prev{0, 0, 0};  // of the counters to clear
+  bool dealt = false;    // this window's rows were dealt again
   for (;;) {
     const float grow = next_grow;
-    const bool last = win + 1 >= a.n_windows;
+    // A deal: a pass with no rotations from this window's bins into better ones.
+    const bool deal = !dealt && first < a.windows[win].n_gates &&
+                      (float)N > REDEAL * (float)SB::R * (float)lay.bins;
+    const bool last = !deal && win + 1 >= a.n_windows;
     const u32 set = ph % 3, nset = (ph + 1) % 3;
     // The rows that will leave this window: as many more or fewer as left the
     // earlier one like it; without one, a reclaim mostly undoes the growth.
     const float* h = alike((float)N, win);
     const float ratio = h ? __ldcg(h + 1) : (a.windows[win].noise == 2 ? 1.0f : 1.5f);
-    const Layout nlay = last ? lay : layout_for((float)N * ratio, win + 1, a.room[(ph + 1) & 1]);
+    const Layout nlay = last ? lay
+                        : deal ? layout_for((float)N, win, a.room[(ph + 1) & 1])
+                               : layout_for((float)N * ratio, win + 1, a.room[(ph + 1) & 1]);
     if (tid == 0) {
       v.w = a.windows[win];
-      v.wn = last ? WinDesc{} : a.windows[win + 1];
+      v.wn = last ? WinDesc{} : a.windows[deal ? win : win + 1];
+      if (deal) v.w.n_gates = v.w.noise = 0;
       if (last) {
         Dest d{};
         d.dense = 1;
@@ -1135,6 +1150,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
       if (grp.bid == 0 && tid == 0) {
         bs->stopped = 1;
         bs->dense_start = 0;
+        bs->dense_end = last ? 1 : 0;
         bs->op = v.w.op + first;
         bs->rows = N;
         bs->phase = ph;
@@ -1147,7 +1163,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
       return;
     }
     const u64 nn = v.y[0];
-    if (grp.bid == 0 && tid == 0) {
+    if (!deal && grp.bid == 0 && tid == 0) {
       if (v.w.noise) a.hist[v.w.op + v.w.n_gates] = nn;
       stamp_op(a.stamps, v.w.op_end - 1);
       if (N && !first) {  // read by windows at least 3 further on
@@ -1156,12 +1172,17 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
         a.growth[3 * win + 2] = (float)N;
       }
     }
-    rho = fmaxf(N ? (float)(N + v.y[1]) / (float)N : 1.0f, 0.85f * rho);
-    N = nn;
     prev = lay;
     lay = nlay;
-    first = 0;
     ++ph;
+    dealt = deal;
+    if (deal) {
+      __syncthreads();  // v is rewritten
+      continue;
+    }
+    rho = fmaxf(N ? (float)(N + v.y[1]) / (float)N : 1.0f, 0.85f * rho);
+    N = nn;
+    first = 0;
     ++win;
     if (win >= a.n_windows) break;
     __syncthreads();  // v is rewritten

@@ -1656,7 +1656,7 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     }
     // The buffer the stopped window was filling (or the dense rows) is grown.
     const u32 fill = hb.dense_start ? 0 : hb.phase + 1;
-    if (!hb.dense_start && P.windows.back().op_end > hb.op && P.windows.back().op <= hb.op) {
+    if (!hb.dense_start && hb.dense_end) {
       if (int rc = E->ensure_dense(S, next_pow2(std::max<u64>(hb.n_dense, S.cap + 1)), 0, W)) return rc;
     } else {
       const u64 want = std::max<u64>(4 * B.room[fill & 1], next_pow2(4 * hb.rows));

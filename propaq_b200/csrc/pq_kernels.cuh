@@ -190,6 +190,7 @@ struct BinState {
   u32 fail[3];     // the set's buffer was too small
   // Where a sweep stopped for a buffer the host has to grow.
   u32 stopped, dense_start;  // dense_start: before any row was dealt
+  u32 dense_end, pad_;       // the buffer is the dense rows the last window writes
   u32 op, phase;   // first op not run; count of buffer fills so far
   u64 rows;
   u32 bins, stride, cap;
