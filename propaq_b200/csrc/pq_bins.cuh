@@ -996,6 +996,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     d.cnt = a.counts + (u64)(set % 3) * a.count_words;
     d.spill_bin = a.spill_bin[set & 1];
     d.room = spill_room(l, a.room[set & 1]);
+    if (a.spill_limit && d.room > spill_limit(a.room[set & 1])) d.room = spill_limit(a.room[set & 1]);
     d.n_spill = &bs->n_spill[set % 3];
     d.n_dense = nullptr;
     d.fail = &bs->fail[set % 3];

@@ -1554,6 +1554,7 @@ int prepare_bins(pq_engine* E, Slot& S, Plan& P, pq::SweepState* st, pq::BinArgs
   a.min_coeff = P.ccut;
   a.n0 = P.n0;
   a.count_words = pq::COUNT_WORDS;
+  a.spill_limit = 1;
   a.growth = S.growth;
   a.born = S.tickets;
   a.anti = S.anti;
@@ -1659,8 +1660,16 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     if (!hb.dense_start && hb.dense_end) {
       if (int rc = E->ensure_dense(S, next_pow2(std::max<u64>(hb.n_dense, S.cap + 1)), 0, W)) return rc;
     } else {
-      const u64 want = std::max<u64>(4 * B.room[fill & 1], next_pow2(4 * hb.rows));
-      if (int rc = E->ensure_bins(B, (int)(fill & 1), want, W)) return rc;
+      const int i = (int)(fill & 1);
+      const u64 have = B.room[i];
+      u64 want = std::max<u64>(4 * have, next_pow2(4 * hb.rows));
+      int rc = E->ensure_bins(B, i, want, W);
+      while (rc == PQ_ERR_OOM && want > 2 * have) rc = E->ensure_bins(B, i, want = std::max(want / 2, 2 * have), W);
+      if (rc == PQ_ERR_OOM && a.spill_limit) {  // as large as it gets: rows may spill as far as there are tags
+        a.spill_limit = 0;
+        rc = E->ensure_bins(B, i, have, W);
+      }
+      if (rc) return rc;
     }
     // Everything the stopped window counted is dropped.
     for (u32 s = 0; s < 3; ++s) {

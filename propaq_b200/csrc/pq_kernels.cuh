@@ -220,6 +220,7 @@ struct BinArgs {
   u64 room[2];        // rows of each buffer
   u32* counts;        // three sets of COUNT_WORDS
   u32 count_words;
+  u32 spill_limit;    // a buffer with more spills than spill_limit() counts as too small
   u32 resume, phase0; // continue a stopped sweep from BinState
   float* growth;      // per window: growth of the live count inside it, rows leaving / entering,
                       // rows entering (0: not run on the grid)

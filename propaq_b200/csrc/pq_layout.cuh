@@ -26,6 +26,11 @@ __host__ __device__ __forceinline__ u64 spill_room(const Layout& l, u64 room) {
   const u64 rest = room - (u64)l.bins * l.cap, tags = spill_tags(room);
   return rest < tags ? rest : tags;
 }
+// Every bin that spilled reads all the tags, so a buffer that more rows than
+// this spill in is grown although it holds them, as long as the device has room
+// for a larger one (2^22 rows in a buffer of 2^22, 260,000 of them spilled: a call
+// that ends in two rotations on them took 5.5 ms, and 1.3 with a larger one).
+__host__ __device__ __forceinline__ u64 spill_limit(u64 room) { return room / 32; }
 
 // Bins for about n rows that a window lets grow by a factor `grow`, grown bins
 // `fill` full.  While a bin of every warp holds at most WARP_ROWS rows when

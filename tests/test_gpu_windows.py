@@ -161,16 +161,16 @@ def test_bins_that_cannot_be_split(gpu_engine, oracle, n):
 
 # -------------------------------------------------- windows that multiply rows
 @pytest.mark.gpu
-@pytest.mark.parametrize("k,n,width,pairs", [(0, 22, 22, ()), (0, 22, 120, ()), (3, 22, 30, (0, 2)),
-                                             (4, 22, 120, (0, 2))],
-                         ids=["W1-2^22", "W4-2^22", "W1-2^25", "W4-2^26"])
+@pytest.mark.parametrize("k,n,width,pairs", [(0, 22, 22, ()), (0, 22, 120, ()), (0, 22, 22, (0, 2)),
+                                             (0, 22, 120, (0, 2)), (3, 22, 30, (0, 2)), (4, 22, 120, (0, 2))],
+                         ids=["W1-2^22", "W4-2^22", "W1-2^22-ZZ", "W4-2^22-ZZ", "W1-2^25-ZZ", "W4-2^26-ZZ"])
 def test_windows_that_multiply_their_rows(k, n, width, pairs):
     # 2^k Z strings under RX on n qubits, then ZZ rotations, against the row
     # sweep (a knob at its default takes it): the same counts and value, and in
     # a time of the same order.  The first two take 0.7 and 0.9 ms on both
     # sweeps (4.1 and 4.6 on the binned one while a pair of groups could send a
-    # block's bins deep), the others 8.7 and 20 ms on the row sweep and 8.0 and
-    # 31 on the binned one (73 and 3,040 before rows were dealt again).
+    # block's bins deep); the last two 8.7 and 20 ms on the row sweep and 8.0
+    # and 31 on the binned one (73 and 3,040 before rows were dealt again).
     rng = np.random.default_rng(k)
     angles = rng.uniform(0.3, 1.2, n)
     x = [PauliRotation(PauliString(1 << q, 0, width), float(angles[q])) for q in range(n)]
