@@ -74,7 +74,7 @@ struct BinSmem {
   u32 n_list[2];                 // their number; the other one is zero for the next rotation
   u32 act[WIN_MAX / 32];         // rotations to run (commuting windows, few rows)
   __align__(8) WinDesc win[4];   // ring (solo): the running window and the next two
-  u32 n;
+  u32 n, quit;
 };
 
 template <class S>
@@ -615,6 +615,7 @@ struct Dest {
   u32* n_spill;    // spilled rows
   u64* n_dense;    // dense (no bins): rows written
   u32* fail;       // set when the buffer is full
+  u32* ticket;     // bins handed out in the window that fills it
   u64 room;        // rows that may spill; dense: rows of the buffer
   Layout l;
   u32 dense;
@@ -676,6 +677,12 @@ __device__ __forceinline__ void load_grouping(WinSmem<W>& v, const BinArgs& a) {
   __syncthreads();
 }
 
+// No further bin is handed out: the window starts again in a larger buffer.
+// The dense rows at the end are all counted first, so they are grown once.
+__device__ __noinline__ void too_small(const Dest& d) {
+  if (!*(volatile u32*)d.fail && !atomicExch(d.fail, 1u) && !d.dense) atomicAdd(d.ticket, NO_MORE_BINS);
+}
+
 template <int W, int ALG>
 __device__ __forceinline__ void put_row(const WinSmem<W>& v, const u64* k, double c, u32 h, bool act,
                                         const GateDesc<W>* gates) {
@@ -690,7 +697,7 @@ __device__ __forceinline__ void put_row(const WinSmem<W>& v, const u64* k, doubl
     at = __shfl_sync(FULL, base, 0) + __popc(m & ((1u << lane) - 1u));
     if (!act) return;
     if (at >= d.room) {
-      *d.fail = 1;
+      too_small(d);
       return;
     }
   } else {
@@ -702,7 +709,7 @@ __device__ __forceinline__ void put_row(const WinSmem<W>& v, const u64* k, doubl
     } else {
       const u32 sp = atomicAdd(d.n_spill, 1u);
       if (sp >= d.room) {
-        *d.fail = 1;
+        too_small(d);
         return;
       }
       at = (u64)d.l.bins * d.l.cap + sp;
@@ -797,6 +804,13 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
   // split at once what would outgrow the unit at the expected growth: failing
   // late in a window of 80 rotations takes as long as running it
   while (!WARP && depth < 24 && (float)(n_all >> depth) * v.grow > (float)S::R * 0.9f) ++depth;
+  // Nothing more is run once the next buffer turned out too small: the window
+  // starts again when the host has grown it.
+  auto given_up = [&] {
+    if (tid == 0) s.quit = !v.d.dense && *(volatile u32*)v.d.fail;
+    unit_sync<S>();
+    return s.quit != 0;
+  };
   const u32 base = depth;
   u32 failed = 0;  // rows of the part that failed last: a half that holds them all fails too
   for (;;) {
@@ -895,7 +909,7 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
         if (tid == 0) atomicOr(&a.st->error, ERR_CAPACITY);
         return true;
       }
-      unit_sync<S>();
+      if (given_up()) return true;
       continue;
     }
     if (n) failed = 0;
@@ -927,6 +941,7 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
       ++depth;
       part <<= 1;
     }
+    if (given_up()) return true;
   }
 }
 
@@ -1000,6 +1015,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     d.n_spill = &bs->n_spill[set % 3];
     d.n_dense = nullptr;
     d.fail = &bs->fail[set % 3];
+    d.ticket = &bs->ticket[(set + 2) % 3];  // of the window before
     return d;
   };
   if (!resumed) {
@@ -1044,6 +1060,14 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     const bool deal = !dealt && first < a.windows[win].n_gates &&
                       (float)N > REDEAL * (float)SB::R * (float)lay.bins;
     const bool last = !deal && win + 1 >= a.n_windows;
+    if (2 * N > a.max_rows && first < a.windows[win].n_gates && a.windows[win].n_basis) {
+      // the first rotation that branches could pass the row ceiling (every block sees the same)
+      if (grp.bid == 0 && tid == 0) {
+        bs->rows = N;
+        atomicOr(&st->error, ERR_CEILING);
+      }
+      return;
+    }
     const u32 set = ph % 3, nset = (ph + 1) % 3;
     // The rows that will leave this window: as many more or fewer as left the
     // earlier one like it; without one, a reclaim mostly undoes the growth.

@@ -28,6 +28,7 @@ enum : u32 {
   ERR_CAPACITY = 4u,          // a write would have passed the row capacity
   ERR_BARRIER_TIMEOUT = 8u,   // a grid barrier wait expired
   ERR_CLASS_FAMILY = 16u,     // a row's family in a class op exceeded CLASS_KMAX (the host rules it out)
+  ERR_CEILING = 32u,          // binned sweep: a rotation could pass the row ceiling (BinState::rows live ones)
 };
 
 __host__ __device__ inline int mod4(int v) { return v & 3; }

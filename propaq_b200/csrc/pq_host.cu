@@ -1555,6 +1555,7 @@ int prepare_bins(pq_engine* E, Slot& S, Plan& P, pq::SweepState* st, pq::BinArgs
   a.n0 = P.n0;
   a.count_words = pq::COUNT_WORDS;
   a.spill_limit = 1;
+  a.max_rows = MAX_ROWS;
   a.growth = S.growth;
   a.born = S.tickets;
   a.anti = S.anti;
@@ -1591,7 +1592,12 @@ void clear_counts(pq_engine* E) {
 // Not an error of the caller's: a bin that no further bit of the group hash
 // splits holds more rows than a block does.  The row sweep runs such a call.
 constexpr int BINS_UNFIT = -1000;
-int bins_error(pq_engine* E, const pq::SweepState& h) {
+int ceiling_reached(pq_engine* E, u64 n) {
+  return E->fail(PQ_ERR_CEILING, "term index ceiling reached: " + std::to_string(2 * n) +
+                                     " rows would exceed the engine's capacity");
+}
+int bins_error(pq_engine* E, const pq::SweepState& h, const pq::BinState& b) {
+  if (h.error == pq::ERR_CEILING) return ceiling_reached(E, b.rows);
   if (h.error == pq::ERR_CAPACITY) return E->fail(BINS_UNFIT, "a bin cannot be split");
   if (h.error & pq::ERR_BARRIER_TIMEOUT)
     return E->fail(PQ_ERR_DEVICE_TIMEOUT, "a grid barrier wait expired on the device");
@@ -1649,7 +1655,7 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     cudaEventElapsedTime(&ms, E->ev_l0, E->ev_l1);
     P.sweep_ms += ms;
     const pq::SweepState& h = E->h_states[0];
-    if (int rc = bins_error(E, h)) return rc;
+    if (int rc = bins_error(E, h, hb)) return rc;
     if (!hb.stopped) {
       P.n_live = h.n[0];
       P.done = no;
@@ -1662,7 +1668,13 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     } else {
       const int i = (int)(fill & 1);
       const u64 have = B.room[i];
+      // the rows of the bins the window had finished when it stopped, for all
+      // its bins (every block took one more ticket, and no bin for it)
+      const u32 tickets = hb.ticket[hb.phase % 3] & (pq::NO_MORE_BINS - 1);
+      double need = hb.dense_start ? 0.0 : (double)hb.n[(hb.phase + 1) % 3];
+      if (tickets > (u32)grid && tickets - grid < hb.bins) need *= (double)hb.bins / (tickets - grid);
       u64 want = std::max<u64>(4 * have, next_pow2(4 * hb.rows));
+      want = std::max(want, next_pow2((u64)std::min(1.125 * need, 2.0 * MAX_ROWS)));
       int rc = E->ensure_bins(B, i, want, W);
       while (rc == PQ_ERR_OOM && want > 2 * have) rc = E->ensure_bins(B, i, want = std::max(want / 2, 2 * have), W);
       if (rc == PQ_ERR_OOM && a.spill_limit) {  // as large as it gets: rows may spill as far as there are tags
@@ -1985,9 +1997,7 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
       u64 n = P.n0;
       for (size_t i = 0; i < no; ++i) {
         const u32 kind = P.ops[i].kind;
-        if (kind == pq::OP_GATE && 2 * n > MAX_ROWS)
-          return E->fail(PQ_ERR_CEILING, "term index ceiling reached: " + std::to_string(2 * n) +
-                                             " rows would exceed the engine's capacity");
+        if (kind == pq::OP_GATE && 2 * n > MAX_ROWS) return ceiling_reached(E, n);
         if (kind == pq::OP_NOISE_COMPACT)
           n = hist[i];
         else if (kind != pq::OP_NOISE_SCALE)
@@ -2456,9 +2466,10 @@ int run_batch_bins(pq_engine* E, std::vector<Plan>& plans) {
   cudaMemcpyAsync(E->h_states, E->d_states, n * sizeof(pq::SweepState), cudaMemcpyDeviceToHost, E->stream);
   if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "solo runs");
   std::vector<u32> rest;
+  std::vector<pq::BinState> hb(n);
   for (size_t i = 0; i < n; ++i) {
     plans[i].sweep_launches = 1;
-    if (int rc = bins_error(E, E->h_states[i])) return rc;
+    if (int rc = bins_error(E, E->h_states[i], hb[i])) return rc;
     if (E->h_states[i].end_op < plans[i].ops.size()) rest.push_back((u32)i);
   }
   for (u32 i : rest) {
@@ -2469,7 +2480,6 @@ int run_batch_bins(pq_engine* E, std::vector<Plan>& plans) {
                   [&](auto w, auto alg) { return pq::launch_bins<w, alg>(args[i], grid[i], E->stream); });
     if (e != cudaSuccess) return E->cuda_fail(e, "binned sweep launch");
   }
-  std::vector<pq::BinState> hb(n);
   if (!rest.empty()) {
     cudaMemcpyAsync(E->h_states, E->d_states, n * sizeof(pq::SweepState), cudaMemcpyDeviceToHost, E->stream);
     for (u32 i : rest)
@@ -2478,7 +2488,7 @@ int run_batch_bins(pq_engine* E, std::vector<Plan>& plans) {
   }
   for (size_t i = 0; i < n; ++i) {
     Plan& P = plans[i];
-    if (int rc = bins_error(E, E->h_states[i])) return rc;
+    if (int rc = bins_error(E, E->h_states[i], hb[i])) return rc;
     P.n_live = E->h_states[i].n[0];
     P.done = P.ops.size();
   }

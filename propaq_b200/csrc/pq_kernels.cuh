@@ -180,6 +180,8 @@ struct BasisDesc {
   u32 pad_;
 };
 
+constexpr u32 NO_MORE_BINS = 1u << 30;  // added to a set's ticket when the buffer being filled is too small
+
 // Device state of a binned sweep; the sets are indexed by window count mod 3.
 struct BinState {
   u64 n[3];        // rows in the set's bins
@@ -218,6 +220,7 @@ struct BinArgs {
   u32* bin_hash[2];
   u32* spill_bin[2];
   u64 room[2];        // rows of each buffer
+  u64 max_rows;       // row ceiling
   u32* counts;        // three sets of COUNT_WORDS
   u32 count_words;
   u32 spill_limit;    // a buffer with more spills than spill_limit() counts as too small
