@@ -115,8 +115,12 @@ typedef struct pq_result {
   double device_ms;           /* device time from the first sweep launch to the
                                  expectation value (CUDA events, engine stream) */
   double sweep_ms;            /* CUDA-event time of the sweep kernel launches  */
-  uint64_t sweep_launches;    /* 1, plus one per capacity growth               */
-  /* Split of the sweep time by op kind, from the device clock at each op's end. */
+  uint64_t sweep_launches;    /* row sweep: 1, plus one per capacity growth and
+                                 per larger grid; binned sweep: a solo and a grid
+                                 launch, plus one per capacity growth           */
+  /* Split of the sweep time by op kind: from the device clock at each op's end
+   * (row sweep), or at the end of a run of rotations and the noise after it,
+   * whose time is shared among its ops by the rows they scan (binned sweep). */
   double gate_ms, noise_ms, phase_ms;
   uint64_t gate_ops, noise_ops, phase_ops;
   uint64_t sum_rows_gate;     /* sum over gate ops of the live rows they scan  */
@@ -212,7 +216,7 @@ typedef struct pq_gate_record {
 
 /* Per-gate records of the last pq_run, gates in Heisenberg order: live
  * counts and device time after every run (a fused op's time goes to its first
- * rotation), the emit statistics (declined, emitted, exchange_hits, the
+ * rotation, the binned sweep's times are shares as in pq_result), the emit statistics (declined, emitted, exchange_hits, the
  * discarded mass) only after a run made with log_gates.  Writes min(cap, n)
  * records, returns n. */
 size_t pq_result_gates(pq_engine* engine, pq_gate_record* out, size_t cap);

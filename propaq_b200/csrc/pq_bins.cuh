@@ -510,7 +510,7 @@ __device__ __noinline__ void solo_run(const BinArgs& a, S& s, u32& win, u32& fir
       if (tid == 0) a.hist[w.op + G] = n;
     }
     // (reading the clock takes about as long as a rotation)
-    if (tid == T - 1 && ((win & 7u) == 7u || win + 1 == a.n_windows)) stamp_op(a.stamps, w.op_end - 1);
+    if (tid == T - 1 && (win & 7u) == 7u) stamp_op(a.stamps, w.op_end - 1);
     if (!met) {
       if (fetcher) cp_async_wait_1();
       unit_sync<S>();
@@ -547,6 +547,7 @@ __device__ __forceinline__ u32 window_of(const BinArgs& a, u32 op) {
 template <int W, int ALG, class SW, class SB>
 __device__ __forceinline__ void solo_body(const BinArgs& a, SW& sw, SB& sb) {
   SweepState* st = a.st;
+  if (threadIdx.x == 0) stamp_op(a.stamps, a.op_end);  // the start
   u32 win = window_of(a, a.op_begin), first = 0, n = 0;
   if (win < a.n_windows && a.op_begin > a.windows[win].op) first = a.op_begin - a.windows[win].op;
   const u64 n0 = a.n0;
@@ -575,8 +576,10 @@ __device__ __forceinline__ void solo_body(const BinArgs& a, SW& sw, SB& sb) {
   }
   if (win < a.n_windows) solo_run<W, ALG>(a, sb, win, first, n);
   if (threadIdx.x == 0) {
+    const u32 end = win < a.n_windows ? a.windows[win].op + first : a.op_end;
     st->n[0] = n;
-    st->end_op = win < a.n_windows ? a.windows[win].op + first : a.op_end;
+    st->end_op = end;
+    if (end > a.op_begin) stamp_op(a.stamps, end - 1);
   }
 }
 
@@ -1019,6 +1022,10 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     return d;
   };
   if (!resumed) {
+    if (grp.bid == 0 && tid == 0) {  // where the grid began
+      stamp_op(a.stamps, a.op_end + 1);
+      a.stamps[a.op_end + 2] = op_start + 1;
+    }
     // Deal the dense rows into the bins of the first window.
     lay = layout_for((float)N, win, a.room[0]);
     if (tid == 0) {

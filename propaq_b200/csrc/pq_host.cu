@@ -627,7 +627,7 @@ struct pq_engine {
     if ((e = dmalloc(&S.d_ops, n_ops * sizeof(pq::OpDesc))) != cudaSuccess ||
         (e = dmalloc(&S.tickets, n_ops * 4)) != cudaSuccess ||
         (e = dmalloc(&S.hist, n_ops * 8)) != cudaSuccess || (e = dmalloc(&S.anti, n_ops * 8)) != cudaSuccess ||
-        (e = dmalloc(&S.stamps, n_ops * 8)) != cudaSuccess ||
+        (e = dmalloc(&S.stamps, (n_ops + 3) * 8)) != cudaSuccess ||
         (e = dmalloc(&S.logs, n_ops * pq::LOG_WORDS * 8)) != cudaSuccess)
       return cuda_fail(e, "allocating op arrays");
     S.ops_cap = n_ops;
@@ -1533,7 +1533,7 @@ int prepare_bins(pq_engine* E, Slot& S, Plan& P, pq::SweepState* st, pq::BinArgs
       cudaMemcpyAsync(S.d_basis, P.basis.data(), P.basis.size() * sizeof(pq::BasisDesc), cudaMemcpyHostToDevice,
                       E->stream);
     cudaMemsetAsync(S.tickets, 0, no * 4, E->stream);
-    cudaMemsetAsync(S.stamps, 0, no * 8, E->stream);
+    cudaMemsetAsync(S.stamps, 0, (no + 3) * 8, E->stream);
   }
   cudaMemsetAsync(S.bin_state, 0, sizeof(pq::BinState) + 3 * nw * sizeof(float), E->stream);
   pq::BinArgs a{};
@@ -1985,15 +1985,18 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
     S.out_keys.resize(n * S.out_words);
   }
   const size_t no = P.ops.size();
-  std::vector<u64> hist(no), anti(no), stamps(no);
+  std::vector<u64> hist(no), anti(no), stamps(no + 3);
+  std::vector<double> op_ms(no, 0.0);
   if (no) {
     cudaMemcpyAsync(hist.data(), S.hist, no * 8, cudaMemcpyDeviceToHost, E->stream);
     cudaMemcpyAsync(anti.data(), S.anti, no * 8, cudaMemcpyDeviceToHost, E->stream);
-    cudaMemcpyAsync(stamps.data(), S.stamps, no * 8, cudaMemcpyDeviceToHost, E->stream);
+    cudaMemcpyAsync(stamps.data(), S.stamps, (no + (P.binned ? 3 : 0)) * 8, cudaMemcpyDeviceToHost, E->stream);
     std::vector<u32> born(P.binned ? no : 0);
     if (P.binned) cudaMemcpyAsync(born.data(), S.tickets, no * 4, cudaMemcpyDeviceToHost, E->stream);
     if (cudaError_t e = cudaStreamSynchronize(E->stream)) return E->cuda_fail(e, "op statistics");
-    if (P.binned) {  // live counts from the rows each rotation created; one stamp per window
+    auto ms = [](u64 from, u64 to) { return to > from ? (double)(to - from) * 1e-6 : 0.0; };
+    for (size_t i = 1; i < no && !P.binned; ++i) op_ms[i] = ms(stamps[i - 1], stamps[i]);
+    if (P.binned) {  // live counts from the rows each rotation created
       u64 n = P.n0;
       for (size_t i = 0; i < no; ++i) {
         const u32 kind = P.ops[i].kind;
@@ -2005,8 +2008,20 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
         hist[i] = n;
         P.peak = std::max(P.peak, n);
       }
-      for (size_t i = no; i-- > 0;)
-        if (!stamps[i] && i + 1 < no) stamps[i] = stamps[i + 1];
+      // One stamp a window, or for several of them solo: its time goes to its
+      // ops by the rows they scan, with 64 rows' worth for an op itself.
+      auto share = [&](size_t k) { return (double)(k ? hist[k - 1] : P.n0) + 64.0; };
+      const size_t grid_op = stamps[no + 2] ? (size_t)stamps[no + 2] - 1 : no;
+      u64 from = stamps[no];
+      for (size_t b = 0, i = 0; i < no; ++i) {
+        if (!stamps[i]) continue;
+        if (b == grid_op) from = stamps[no + 1];
+        double all = 0;
+        for (size_t k = b; k <= i; ++k) all += share(k);
+        for (size_t k = b; k <= i; ++k) op_ms[k] = ms(from, stamps[i]) * share(k) / all;
+        from = stamps[i];
+        b = i + 1;
+      }
     }
   }
   if (in.n_terms_out)
@@ -2037,14 +2052,13 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
             std::memcpy(&rcd.discarded_coeff_max, &w[pq::LOG_MAX], 8);
           }
           // the op's device time; a fused op's time goes to its first rotation
-          rcd.elapsed_ms = op > 0 && stamps[op] > stamps[op - 1] ? (double)(stamps[op] - stamps[op - 1]) * 1e-6 : 0.0;
+          rcd.elapsed_ms = op_ms[op];
         }
       }
   }
   for (size_t i = 0; i < no; ++i) {
     if (pq::is_class(P.ops[i].kind)) ++res->class_ops;
     const u64 n_in = i ? hist[i - 1] : P.n0;
-    const double op_ms = i && stamps[i] > stamps[i - 1] ? (double)(stamps[i] - stamps[i - 1]) * 1e-6 : 0.0;
     switch (pq::is_class(P.ops[i].kind) ? (u32)pq::OP_GATE : P.ops[i].kind) {
       case pq::OP_GATE:
       case pq::OP_GATE2:
@@ -2052,19 +2066,19 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
       case pq::OP_GATE4:
       case pq::OP_GATE_TAIL:
         ++res->gate_ops;
-        res->gate_ms += op_ms;
+        res->gate_ms += op_ms[i];
         res->sum_rows_gate += n_in;
         res->sum_anti += anti[i];
         res->sum_children += hist[i] - n_in;
         break;
       case pq::OP_PHASE:
         ++res->phase_ops;
-        res->phase_ms += op_ms;
+        res->phase_ms += op_ms[i];
         res->sum_rows_phase += n_in;
         break;
       default:
         ++res->noise_ops;
-        res->noise_ms += op_ms;
+        res->noise_ms += op_ms[i];
         res->sum_rows_noise += n_in;
         res->sum_kept += P.ops[i].kind == pq::OP_NOISE_COMPACT ? hist[i] : 0;
     }

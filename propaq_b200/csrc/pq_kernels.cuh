@@ -230,7 +230,8 @@ struct BinArgs {
   u32* born;          // per op: rows created
   u64* anti;          // per op: rows anticommuting
   u64* hist;          // noise ops: live count after
-  u64* stamps;        // device clock at the end of a window (its last op) / a solo op
+  u64* stamps;        // device clock at the last op of a window, or of several solo ones; then at
+                      // [op_end] of the solo start, [op_end + 1] of the grid's, [op_end + 2] its first op + 1
   SweepState* st;
   BinState* bs;
   u32 hold_block, hold_us;
