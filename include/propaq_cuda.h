@@ -107,7 +107,9 @@ typedef struct pq_run_config {
 typedef struct pq_result {
   double expectation_value;   /* 0 when no diag_state was given               */
   uint64_t terms_below_cutoff;/* live terms with |c| < min_coeff at the end   */
-  uint64_t sparse_key_bytes;  /* device bytes holding keys and the hash table */
+  uint64_t sparse_key_bytes;  /* device bytes holding the final terms' keys, and
+                                 the row sweep's hash table (the binned sweep
+                                 keeps its tables in shared memory)             */
   uint64_t n_final;           /* live terms at the end                        */
   uint64_t n_layers_run, n_gates_run;
   uint64_t gpu_launches;      /* kernels this run launched                    */

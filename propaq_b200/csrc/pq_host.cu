@@ -2089,7 +2089,7 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
   res->n_final = P.n_live;
   res->peak_terms = P.peak;
   S.seen_rows = std::max(S.seen_rows, P.peak);
-  res->sparse_key_bytes = P.n_live * P.W * 8 + S.tcap * 8;
+  res->sparse_key_bytes = P.n_live * P.W * 8 + (P.binned ? 0 : S.tcap * 8);
   res->n_layers_run = in.n_layers;
   res->n_gates_run = in.n_gates;
   return PQ_OK;
