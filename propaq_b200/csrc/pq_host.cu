@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <string>
 #include <type_traits>
@@ -150,6 +151,7 @@ u64 next_pow2(u64 x) {
 struct MemBudget {
   size_t limit = 0, used = 0;  // limit 0 = none
   std::unordered_map<void*, size_t> sizes;
+  std::function<bool()> release_idle;  // frees buffers that hold nothing; false if there were none
 };
 thread_local MemBudget* t_budget = nullptr;
 
@@ -163,9 +165,16 @@ template <class T>
 cudaError_t dmalloc(T** p, size_t n) {
   *p = nullptr;
   MemBudget* b = t_budget;
-  if (b && b->limit && b->used + n > b->limit) return cudaErrorMemoryAllocation;
   void* q = nullptr;
-  const cudaError_t e = cudaMalloc(&q, n);
+  auto attempt = [&] {
+    if (b && b->limit && b->used + n > b->limit) return cudaErrorMemoryAllocation;
+    return cudaMalloc(&q, n);
+  };
+  cudaError_t e = attempt();
+  if (e == cudaErrorMemoryAllocation && b && b->release_idle && b->release_idle()) {
+    cudaGetLastError();
+    e = attempt();
+  }
   if (e != cudaSuccess) return e;
   *p = static_cast<T*>(q);
   if (b) {
@@ -417,6 +426,7 @@ struct pq_engine {
   DevBuf g_pool, g_lam, g_ops;
   u32* d_lin = nullptr;  // linear hash tables of the binned sweep
   pq::BinState* h_bins = nullptr;  // pinned
+  bool bins_used = false;  // a binned sweep is running: its buffers hold rows
   DevBuf batch_args;  // arguments of a binned batch's solo runs
   DevBuf sort_buf;  // radix-sort scratch and sorted rows (observable folding, sorted term output)
   std::vector<DevBuf> g_ck;
@@ -467,6 +477,20 @@ struct pq_engine {
     for (auto ev : {ev_begin, ev_end, ev_l0, ev_l1})
       if (ev) cudaEventDestroy(ev);
     if (stream) cudaStreamDestroy(stream);
+  }
+  // The bin buffers between binned sweeps: given back to any allocation of the
+  // engine's that finds no room beside them.
+  size_t idle_bin_bytes() const {
+    if (bins_used || slots.empty()) return 0;
+    size_t n = 0;
+    for (int i = 0; i < 2; ++i)
+      n += slots[0].bin_words[i] * 8 + slots[0].bin_rows[i] * 12 + pq::spill_tags(slots[0].bin_rows[i]) * 4;
+    return n;
+  }
+  bool release_idle_bins() {
+    if (!idle_bin_bytes()) return false;
+    for (int i = 0; i < 2; ++i) slots[0].free_bins(i);
+    return true;
   }
   int ensure_slots(size_t n) {
     if (slots.size() < n) slots.resize(n);
@@ -2116,7 +2140,9 @@ int run_one(pq_engine* E, const Inputs& in, int W, bool bins = true) {
   if (int rc = build_ops(P, need_n)) return rc;
   if (P.binned) {
     plan_windows(P);
+    E->bins_used = true;
     const int rc = execute_bins(E, S, P, &began);
+    E->bins_used = false;
     if (rc == PQ_ERR_OOM) {  // the row sweep may still fit
       S.free_bins(0);
       S.free_bins(1);
@@ -2191,6 +2217,7 @@ int run_adjoint(pq_engine* E, const Inputs& in, int W, u32 ckpt_layers, u64 reco
   // most 48 GB).  The engine keeps it for the next gradient.
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
+  free_b += E->idle_bin_bytes();
   const size_t ceiling = std::min<size_t>((free_b + E->g_pool.bytes) / 5 * 2, (size_t)48 << 30);
   Recording rec;
   auto setup_pool = [&](size_t budget) -> cudaError_t {
@@ -2573,7 +2600,9 @@ int run_batch(pq_engine* E, const std::vector<Inputs>& ins, int WM, const pq_bat
     upload_ops(E, E->slots[i], plans[i]);
   }
   if (binned) {
+    E->bins_used = true;
     const int rc = run_batch_bins(E, plans);
+    E->bins_used = false;
     if (rc == PQ_ERR_OOM) {  // the row sweep may still fit
       E->slots[0].free_bins(0);
       E->slots[0].free_bins(1);
@@ -2680,6 +2709,7 @@ int pq_engine_create(pq_engine** out, int device) {
   E->expect_grid = 4 * sms;
   for (cudaEvent_t* ev : {&E->ev_begin, &E->ev_end, &E->ev_l0, &E->ev_l1}) cudaEventCreate(ev);
   if (E->ensure_slots(1) != PQ_OK) return PQ_ERR_OOM;
+  E->budget.release_idle = [engine = E.get()] { return engine->release_idle_bins(); };
   *out = E.release();
   return PQ_OK;
 }
