@@ -959,7 +959,7 @@ int setup_slot(pq_engine* E, Slot& S, Plan& P) {
   }
   cudaMemsetAsync(S.anti, 0, n_ops_max * 8, E->stream);
   if (P.log) cudaMemsetAsync(S.logs, 0, n_ops_max * pq::LOG_WORDS * 8, E->stream);
-  if (S.epoch_base > (1u << 29)) {  // keep status tags unique: restart the epochs on a cleared array
+  if (!P.binned && S.epoch_base > (1u << 29)) {  // keep status tags unique: restart the epochs on a cleared array
     S.epoch_base = 1;
     cudaMemsetAsync(S.status, 0, (S.cap / TILE_ROWS + 2) * 8, E->stream);
   }

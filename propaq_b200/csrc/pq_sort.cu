@@ -11,9 +11,13 @@
 //
 // A pass is three kernels:
 //   digit_count    per block, the rows of its tile holding each digit value;
-//   count_scan     one block: the exclusive scan of those counts taken digit
-//                  major (every block's count of digit 0, then of digit 1 ...),
-//                  which is where each (digit, block) run starts in the output;
+//   digit_scan     a block per digit: the exclusive scan of those counts taken
+//                  digit major (every block's count of digit 0, then of digit 1
+//                  ...), which is where each (digit, block) run starts in the
+//                  output.  A digit's first run starts after the rows of lower
+//                  digits, which the tally holds, so the digits are independent;
+//                  one block over all counts took 0.88 of the 0.94 ms of a
+//                  pass over 2^22 rows, a block per digit takes 0.008;
 //   digit_scatter  per block, its tile again, 256 rows at a time: a row's place
 //                  is its run's start plus the rows of equal digit before it
 //                  (earlier 256-row chunks, earlier warps, earlier lanes:
@@ -97,6 +101,44 @@ __global__ void __launch_bounds__(1024) count_scan_kernel(u32* counts, u64 m) {
     const u32 v = counts[i];
     counts[i] = run;
     run += v;
+  }
+}
+
+// The counts of digit blockIdx.x (nblk of them) replaced by where their runs
+// start; tally: rows of each digit.
+template <int T>
+__global__ void __launch_bounds__(T) digit_scan_kernel(u32* counts, u32 nblk, const u32* tally) {
+  __shared__ u32 part[T / 32];
+  const u32 d = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // exclusive scan over the block; *all receives the total
+  auto scan = [&](u32 v, u32* all) {
+    u32 s = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(FULL_MASK, s, o);
+      if (lane >= o) s += y;
+    }
+    if (lane == 31) part[warp] = s;
+    __syncthreads();
+    u32 before = 0, t = 0;
+#pragma unroll
+    for (int w = 0; w < T / 32; ++w) {
+      if (w == warp) before = t;
+      t += part[w];
+    }
+    __syncthreads();
+    *all = t;
+    return before + s - v;
+  };
+  u32 run = 0, all;
+  scan(threadIdx.x < d ? tally[threadIdx.x] : 0u, &run);
+  u32* c = counts + (u64)d * nblk;
+  for (u32 i0 = 0; i0 < nblk; i0 += T) {
+    const u32 i = i0 + threadIdx.x;
+    const u32 at = scan(i < nblk ? c[i] : 0u, &all);
+    if (i < nblk) c[i] = run + at;
+    run += all;
   }
 }
 
@@ -214,7 +256,8 @@ cudaError_t sort_rows(const u64* keys, const double* coeffs, u64 n, u64* keys_ou
     u64* dk = to_out ? keys_out : tk;
     double* dc = to_out ? coeffs_out : tc;
     digit_count_kernel<W><<<nblk, SORT_BLOCK, 0, s>>>(src_k, n, passes[i], counts, nblk);
-    count_scan_kernel<<<1, 1024, 0, s>>>(counts, m);
+    if (nblk <= 1024) digit_scan_kernel<256><<<256, 256, 0, s>>>(counts, nblk, tally + passes[i] * 256);
+    else digit_scan_kernel<1024><<<256, 1024, 0, s>>>(counts, nblk, tally + passes[i] * 256);
     digit_scatter_kernel<W><<<nblk, SORT_BLOCK, 0, s>>>(src_k, src_c, n, passes[i], counts, nblk, dk, dc);
     *launches += 3;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
