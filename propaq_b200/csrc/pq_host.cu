@@ -286,6 +286,7 @@ struct Slot {
   int out_words = 0;  // width of out_keys (the caller's width)
   std::vector<u64> out_keys;
   std::vector<double> out_coeffs;
+  bool sort_out = false;  // out_keys / out_coeffs are still to be sorted, on the host
 
   void free_rows() {
     for (int i = 0; i < 2; ++i) {
@@ -1943,6 +1944,7 @@ int finalize(pq_engine* E, Slot& S, Plan& P, std::vector<pq::ExpectPartial>* par
   S.out_keys.clear();
   S.out_coeffs.clear();
   S.out_words = in.in_words;
+  S.sort_out = false;
   if (in.cfg->want_terms && n_fin) {
     S.out_keys.resize(n_fin * W);
     S.out_coeffs.resize(n_fin);
@@ -1960,22 +1962,48 @@ int finalize(pq_engine* E, Slot& S, Plan& P, std::vector<pq::ExpectPartial>* par
     const double* out_c = S.coeffs[src];
     if (in.cfg->want_terms == 2 || P.binned) {  // in key order (bins hold rows in no fixed order): the radix sort into the engine's sort buffer
       const u64 sw = pq::sort_scratch_words(n_fin, W);
-      if ((e = E->sort_buf.ensure((sw + n_fin * (u64)(W + 1)) * 8)) != cudaSuccess)
+      e = E->sort_buf.ensure((sw + n_fin * (u64)(W + 1)) * 8);
+      if (e == cudaErrorMemoryAllocation && in.cfg->want_terms != 2) {  // no key order was asked for, only a fixed one
+        cudaGetLastError();
+        S.sort_out = true;
+      } else if (e != cudaSuccess) {
         return E->cuda_fail(e, "sort scratch");
-      u64* scratch = E->sort_buf.at<u64>(0);
-      u64* sk = scratch + sw;
-      double* sc = reinterpret_cast<double*>(sk + n_fin * W);
-      e = with_words(W, [&](auto w) {
-        return pq::sort_rows<decltype(w)::value>(out_k, out_c, n_fin, sk, sc, scratch, E->stream, &E->launches);
-      });
-      if (e != cudaSuccess) return E->cuda_fail(e, "sorting the terms");
-      out_k = sk;
-      out_c = sc;
+      } else {
+        u64* scratch = E->sort_buf.at<u64>(0);
+        u64* sk = scratch + sw;
+        double* sc = reinterpret_cast<double*>(sk + n_fin * W);
+        e = with_words(W, [&](auto w) {
+          return pq::sort_rows<decltype(w)::value>(out_k, out_c, n_fin, sk, sc, scratch, E->stream, &E->launches);
+        });
+        if (e != cudaSuccess) return E->cuda_fail(e, "sorting the terms");
+        out_k = sk;
+        out_c = sc;
+      }
     }
     cudaMemcpyAsync(S.out_keys.data(), out_k, n_fin * W * 8, cudaMemcpyDeviceToHost, E->stream);
     cudaMemcpyAsync(S.out_coeffs.data(), out_c, n_fin * 8, cudaMemcpyDeviceToHost, E->stream);
   }
   return PQ_OK;
+}
+
+// Terms into key order (word W-1 most significant), where the device had no
+// room to sort them.
+void sort_terms(int W, std::vector<u64>& keys, std::vector<double>& coeffs) {
+  std::vector<u64> at(coeffs.size());
+  for (size_t i = 0; i < at.size(); ++i) at[i] = i;
+  std::sort(at.begin(), at.end(), [&](u64 a, u64 b) {
+    for (int w = W; w-- > 0;)
+      if (keys[a * W + w] != keys[b * W + w]) return keys[a * W + w] < keys[b * W + w];
+    return false;
+  });
+  std::vector<u64> k(keys.size());
+  std::vector<double> c(coeffs.size());
+  for (size_t i = 0; i < at.size(); ++i) {
+    std::copy_n(&keys[at[i] * W], W, &k[i * W]);
+    c[i] = coeffs[at[i]];
+  }
+  keys.swap(k);
+  coeffs.swap(c);
 }
 
 // Host half of the result, once the stream has drained: the double-double
@@ -2002,6 +2030,7 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
     if (in.diag) res->expectation_value = hi + lo;
     res->terms_below_cutoff = P.has_c ? below : 0;
   }
+  if (S.sort_out) sort_terms(P.W, S.out_keys, S.out_coeffs);
   if (S.out_words < P.W && !S.out_coeffs.empty()) {  // drop the zero words the device width added
     const size_t n = S.out_coeffs.size();
     for (size_t i = 0; i < n; ++i)

@@ -3,11 +3,15 @@ ran before it."""
 
 from __future__ import annotations
 
+import gc
+
 import numpy as np
 import pytest
-from harness import assert_terms_equal, from_workload, make_cfg, run_gpu, run_oracle
+from harness import assert_terms_equal, from_circuit, from_workload, make_cfg, run_gpu, run_oracle
 
 from propaq_b200 import _native, workloads
+from propaq_b200.circuits import PauliCircuit, PauliRotation
+from propaq_b200.datatypes import PauliString, PauliTermSum
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +53,28 @@ def test_idle_bins_make_room_for_other_runs(oracle):
     g = run_gpu(engine, p)
     assert np.array_equal(g.n_terms, o.n_terms)
     assert_terms_equal(g.keys, g.coeffs, o.keys, o.coeffs)
+
+
+def test_terms_without_room_to_sort_them():
+    # 2^21 terms of 4 words.  With next to no device memory left, the scratch
+    # their sort takes (150 MB and more) is not there even with the idle bins
+    # given back, and the host sorts them: the same terms in the same order.
+    import torch
+
+    n, width = 21, 120
+    rng = np.random.default_rng(3)
+    x = [PauliRotation(PauliString(1 << q, 0, width), float(a)) for q, a in enumerate(rng.uniform(0.3, 1.2, n))]
+    p = from_circuit(0, width, PauliTermSum({PauliString(0, (1 << n) - 1, width): 1.0}), PauliCircuit([x]), 0)
+    want = run_gpu(_native.Engine(0), p)
+    engine = _native.Engine(0)
+    run(engine, p)
+    gc.collect()
+    free = torch.cuda.mem_get_info()[0]
+    held = torch.empty(free - (4 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        g = run_gpu(engine, p)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert g.n_final == 1 << n
+    assert np.array_equal(g.keys, want.keys) and np.array_equal(g.coeffs, want.coeffs)
