@@ -1339,11 +1339,11 @@ void plan_windows(Plan& P) {
       // Rotations on disjoint qubits commute, but a phase rotation may lie
       // across any of them, in a disjoint window too.
       w.commute = 1;
-      auto phase = [&](size_t k) { return P.ops[i + k].kind == pq::OP_PHASE; };
-      for (size_t x = 1; x < len && w.commute; ++x)
-        for (size_t y = 0; y < x && w.commute; ++y)
-          if ((!w.disjoint || phase(x) || phase(y)) && host_anticommutes(P.alg, W, gen(i + x), gen(i + y)))
-            w.commute = 0;
+      for (size_t x = 0; x < len && w.commute; ++x) {
+        if (w.disjoint && P.ops[i + x].kind != pq::OP_PHASE) continue;
+        for (size_t y = 0; y < (w.disjoint ? len : x) && w.commute; ++y)
+          if (host_anticommutes(P.alg, W, gen(i + x), gen(i + y))) w.commute = 0;
+      }
       i += len;
     }
     w.n_basis = (u32)P.basis.size() - w.basis;
