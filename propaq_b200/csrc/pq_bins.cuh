@@ -948,13 +948,70 @@ __device__ __forceinline__ bool run_bin(const BinArgs& a, WinSmem<W>& v, S& s, u
   }
 }
 
-// A layout is made before the window that fills it has run.  Rows that came
-// to more than this many times what its bins hold are dealt again first, by
-// their actual number: one pass over the rows, where bins that are split into
-// four parts and more are read as many times.  (From 2^26 rows on in the bins
-// of a few thousand, the two rotations after a doubling window took 3,031 ms
-// of 4-word keys and 64 of 1-word keys; the runs around them now take 31 and 8.)
+// Bins of fill number `fill` (buffer fill & 1, counter set fill % 3) as a destination.
+__device__ __forceinline__ Dest dest_bins(const BinArgs& a, u32 fill, const Layout& l) {
+  BinState* bs = a.bs;
+  Dest d;
+  d.dense = 0;
+  d.l = l;
+  d.keys = a.bin_keys[fill & 1];
+  d.coeffs = a.bin_coeffs[fill & 1];
+  d.h = a.bin_hash[fill & 1];
+  d.cnt = a.counts + (u64)(fill % 3) * a.count_words;
+  d.spill_bin = a.spill_bin[fill & 1];
+  d.room = spill_room(l, a.room[fill & 1]);
+  if (a.spill_limit && d.room > spill_limit(a.room[fill & 1])) d.room = spill_limit(a.room[fill & 1]);
+  d.n_spill = &bs->n_spill[fill % 3];
+  d.n_dense = nullptr;
+  d.fail = &bs->fail[fill % 3];
+  d.ticket = &bs->ticket[(fill + 2) % 3];  // of the window before
+  return d;
+}
+
+// A layout is made before the window that fills it has run.  A sweep whose
+// rows came to more than this many times what their bins hold stops, and they
+// are dealt again by their actual number (deal_body): one pass over the rows,
+// where bins that are split into four parts and more are read as many times.
+// (On 2^26 rows of 4-word keys and 2^25 of 1-word keys in the bins of a few
+// thousand, the two rotations after a doubling window took 3,031 and 64 ms;
+// the calls around them now take 22 and 8.)  A kernel of its own: a pass of
+// this kind inside bins_body cost the 24-site Givens circuit 4% (10.95 ->
+// 11.41 ms) in registers that every window's rotations need.
 constexpr float REDEAL = 2.0f;
+
+// The rows of the bins `from`, fill number `fill`, into the bins `to` of the
+// next fill, grouped for window `win`.
+template <int W, int ALG, int T>
+__device__ __forceinline__ void deal_body(const BinArgs& a, WinSmem<W>& v, u32 win, u32 fill, const Layout& from,
+                                          const Layout& to) {
+  const int tid = threadIdx.x;
+  const GateDesc<W>* gates = reinterpret_cast<const GateDesc<W>*>(a.gates);
+  if (tid == 0) {
+    v.wn = a.windows[win];
+    v.d = dest_bins(a, fill + 1, to);
+  }
+  __syncthreads();
+  load_grouping<W>(v, a);
+  auto put = [&](u64 src, bool act) {
+    u64 k[W];
+    double c = 0.0;
+    u32 h = 0;
+    if (act) {
+      load_key<W>(a.bin_keys[fill & 1], src, k);
+      c = __ldcg(a.bin_coeffs[fill & 1] + src);
+      h = __ldcg(a.bin_hash[fill & 1] + src);
+    }
+    put_row<W, ALG>(v, k, c, h, act, gates);
+  };
+  const u32* cnt = a.counts + (u64)(fill % 3) * a.count_words;
+  for (u32 b = blockIdx.x; b < from.bins; b += gridDim.x) {
+    const u32 all = __ldcg(cnt + (u64)b * from.stride), n = all < from.cap ? all : from.cap;
+    for (u32 r0 = 0; r0 < n; r0 += T) put((u64)b * from.cap + r0 + tid, r0 + tid < n);
+  }
+  const u32 spilled = a.bs->n_spill[fill % 3];
+  for (u64 r0 = (u64)blockIdx.x * T; r0 < spilled; r0 += (u64)gridDim.x * T)
+    put((u64)from.bins * from.cap + r0 + tid, r0 + tid < spilled);
+}
 
 // The windows from where the solo run (or a stopped sweep) left off, by the
 // blocks of grp.  SB: a block's rows, SW: a warp's; both lie over one another
@@ -1004,23 +1061,6 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     const float fill = h ? (g < 3.0f ? 0.85f : 0.3f) : (a.windows[x].n_gates < 24 ? 1.0f : 0.7f);
     return choose_layout(n, g, fill, grp.nblk, WARPS, SB::R, room);
   };
-  auto dest_bins = [&](u32 set, const Layout& l) {
-    Dest d;
-    d.dense = 0;
-    d.l = l;
-    d.keys = a.bin_keys[set & 1];
-    d.coeffs = a.bin_coeffs[set & 1];
-    d.h = a.bin_hash[set & 1];
-    d.cnt = a.counts + (u64)(set % 3) * a.count_words;
-    d.spill_bin = a.spill_bin[set & 1];
-    d.room = spill_room(l, a.room[set & 1]);
-    if (a.spill_limit && d.room > spill_limit(a.room[set & 1])) d.room = spill_limit(a.room[set & 1]);
-    d.n_spill = &bs->n_spill[set % 3];
-    d.n_dense = nullptr;
-    d.fail = &bs->fail[set % 3];
-    d.ticket = &bs->ticket[(set + 2) % 3];  // of the window before
-    return d;
-  };
   if (!resumed) {
     if (grp.bid == 0 && tid == 0) {  // where the grid began
       stamp_op(a.stamps, a.op_end + 1);
@@ -1030,7 +1070,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     lay = layout_for((float)N, win, a.room[0]);
     if (tid == 0) {
       v.wn = a.windows[win];
-      v.d = dest_bins(0, lay);
+      v.d = dest_bins(a, 0, lay);
     }
     __syncthreads();
     load_grouping<W>(v, a);
@@ -1050,7 +1090,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     if (*(volatile u32*)&st->error) return;
     if (*(volatile u32*)&bs->fail[0]) {  // the first buffer is too small: the dense rows are untouched
       if (grp.bid == 0 && tid == 0) {
-        bs->stopped = 1;
+        bs->stopped = STOP_GROW;
         bs->dense_start = 1;
         bs->op = op_start;
         bs->rows = N;
@@ -1060,13 +1100,29 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
   }
 
   Layout prev{0, 0, 0};  // of the counters to clear
-  bool dealt = false;    // this window's rows were dealt again
+  // Where a launch ends before the last window, for the host to go on from.
+  auto stop = [&](u32 why, bool dense_end, float grow) {
+    if (grp.bid != 0 || tid != 0) return;
+    bs->stopped = why;
+    bs->dense_start = 0;
+    bs->dense_end = dense_end;
+    bs->op = a.windows[win].op + first;
+    bs->rows = N;
+    bs->phase = ph;
+    bs->bins = lay.bins;
+    bs->stride = lay.stride;
+    bs->cap = lay.cap;
+    bs->rho = rho;
+    bs->grow = grow;
+  };
   for (;;) {
     const float grow = next_grow;
-    // A deal: a pass with no rotations from this window's bins into better ones.
-    const bool deal = !dealt && first < a.windows[win].n_gates &&
-                      (float)N > REDEAL * (float)SB::R * (float)lay.bins;
-    const bool last = !deal && win + 1 >= a.n_windows;
+    const bool last = win + 1 >= a.n_windows;
+    if ((float)N > REDEAL * (float)SB::R * (float)lay.bins && first < a.windows[win].n_gates &&
+        a.windows[win].op + first != a.dealt_op) {
+      stop(STOP_DEAL, false, grow);
+      return;
+    }
     if (2 * N > a.max_rows && first < a.windows[win].n_gates && a.windows[win].n_basis) {
       // the first rotation that branches could pass the row ceiling (every block sees the same)
       if (grp.bid == 0 && tid == 0) {
@@ -1080,13 +1136,10 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     // earlier one like it; without one, a reclaim mostly undoes the growth.
     const float* h = alike((float)N, win);
     const float ratio = h ? __ldcg(h + 1) : (a.windows[win].noise == 2 ? 1.0f : 1.5f);
-    const Layout nlay = last ? lay
-                        : deal ? layout_for((float)N, win, a.room[(ph + 1) & 1])
-                               : layout_for((float)N * ratio, win + 1, a.room[(ph + 1) & 1]);
+    const Layout nlay = last ? lay : layout_for((float)N * ratio, win + 1, a.room[(ph + 1) & 1]);
     if (tid == 0) {
       v.w = a.windows[win];
-      v.wn = last ? WinDesc{} : a.windows[deal ? win : win + 1];
-      if (deal) v.w.n_gates = v.w.noise = 0;
+      v.wn = last ? WinDesc{} : a.windows[win + 1];
       if (last) {
         Dest d{};
         d.dense = 1;
@@ -1097,7 +1150,7 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
         d.fail = &bs->fail[nset];
         v.d = d;
       } else {
-        v.d = dest_bins(ph + 1, nlay);
+        v.d = dest_bins(a, ph + 1, nlay);
       }
       v.bk = a.bin_keys[ph & 1];
       v.bc = a.bin_coeffs[ph & 1];
@@ -1179,23 +1232,11 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
     __syncthreads();
     if (v.x[0]) return;
     if (v.x[1]) {  // the next buffer was too small: this window is run again after the host has grown it
-      if (grp.bid == 0 && tid == 0) {
-        bs->stopped = 1;
-        bs->dense_start = 0;
-        bs->dense_end = last ? 1 : 0;
-        bs->op = v.w.op + first;
-        bs->rows = N;
-        bs->phase = ph;
-        bs->bins = lay.bins;
-        bs->stride = lay.stride;
-        bs->cap = lay.cap;
-        bs->rho = rho;
-        bs->grow = grow;
-      }
+      stop(STOP_GROW, last, grow);
       return;
     }
     const u64 nn = v.y[0];
-    if (!deal && grp.bid == 0 && tid == 0) {
+    if (grp.bid == 0 && tid == 0) {
       if (v.w.noise) a.hist[v.w.op + v.w.n_gates] = nn;
       stamp_op(a.stamps, v.w.op_end - 1);
       if (N && !first) {  // read by windows at least 3 further on
@@ -1204,17 +1245,12 @@ __device__ __forceinline__ void bins_body(const BinArgs& a, const Grp grp, WinSm
         a.growth[3 * win + 2] = (float)N;
       }
     }
-    prev = lay;
-    lay = nlay;
-    ++ph;
-    dealt = deal;
-    if (deal) {
-      __syncthreads();  // v is rewritten
-      continue;
-    }
     rho = fmaxf(N ? (float)(N + v.y[1]) / (float)N : 1.0f, 0.85f * rho);
     N = nn;
+    prev = lay;
+    lay = nlay;
     first = 0;
+    ++ph;
     ++win;
     if (win >= a.n_windows) break;
     __syncthreads();  // v is rewritten

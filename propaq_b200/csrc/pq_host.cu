@@ -1581,6 +1581,7 @@ int prepare_bins(pq_engine* E, Slot& S, Plan& P, pq::SweepState* st, pq::BinArgs
   a.count_words = pq::COUNT_WORDS;
   a.spill_limit = 1;
   a.max_rows = MAX_ROWS;
+  a.dealt_op = 0xffffffffu;
   a.growth = S.growth;
   a.born = S.tickets;
   a.anti = S.anti;
@@ -1633,6 +1634,68 @@ int bins_error(pq_engine* E, const pq::SweepState& h, const pq::BinState& b) {
 int bins_grid_for(pq_engine* E, const Plan& P, int* grid) {
   *grid = with_bins(P.W, P.alg, [](auto w, auto alg) { return pq::bins_grid<w, alg>(); });
   return *grid > 0 ? PQ_OK : E->fail(PQ_ERR_CUDA, "the binned sweep does not fit this device");
+}
+
+// Bin buffer i grown to `want` rows, or as far towards that as there is memory.
+int grow_bins(pq_engine* E, pq::BinArgs& a, int i, u64 want, int W) {
+  Slot& B = E->slots[0];
+  const u64 have = B.room[i];
+  int rc = E->ensure_bins(B, i, want, W);
+  while (rc == PQ_ERR_OOM && want > 2 * have) rc = E->ensure_bins(B, i, want = std::max(want / 2, 2 * have), W);
+  if (rc == PQ_ERR_OOM && a.spill_limit) {  // as large as it gets: rows may spill as far as there are tags
+    a.spill_limit = 0;
+    rc = E->ensure_bins(B, i, have, W);
+  }
+  return rc;
+}
+
+// A sweep that stopped for it (STOP_DEAL): the rows into bins that hold them,
+// laid out by their number and the growth of the windows before; the sweep
+// goes on from there.  hb is the stopped sweep's state, as it is on the device.
+int deal_bins(pq_engine* E, Slot& S, const Plan& P, pq::BinArgs& a, pq::BinState& hb, int grid) {
+  cudaError_t e;
+  Slot& B = E->slots[0];
+  const int W = P.W;
+  u32 win = 0;
+  while (P.windows[win].op_end <= hb.op) ++win;
+  const u32 set = hb.phase % 3, next = (hb.phase + 1) % 3;
+  const int i = (int)((hb.phase + 1) & 1);
+  const pq::Layout from{hb.bins, hb.stride, hb.cap};
+  const float g = std::min(std::max(1.15f * hb.rho, 1.5f), 3.0f);
+  const u32 rows = with_bins(W, 0, [](auto w, auto) { return pq::bin_rows<w>(); });
+  auto clear = [&](u32 s) {
+    cudaMemsetAsync(B.counts + (size_t)s * pq::COUNT_WORDS, 0, (size_t)pq::COUNT_WORDS * 4, E->stream);
+    for (u32 x = 0; x < 3; ++x) hb.ticket[x] = hb.fail[x] = 0;
+    hb.n_spill[s] = 0;
+  };
+  pq::Layout to{};
+  for (;;) {
+    bind_bins(E, S, a);
+    to = pq::choose_layout((float)hb.rows, g, P.windows[win].n_gates < 24 ? 1.0f : 0.7f, (u32)grid,
+                           pq::BIN_THREADS / 32, rows, B.room[i]);
+    ++E->launches;
+    e = with_bins(W, P.alg,
+                  [&](auto w, auto alg) { return pq::launch_deal<w, alg>(a, win, hb.phase, from, to, grid, E->stream); });
+    if (e != cudaSuccess) return E->cuda_fail(e, "deal launch");
+    cudaMemcpyAsync(&hb, S.bin_state, sizeof hb, cudaMemcpyDeviceToHost, E->stream);
+    if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "dealing rows again");
+    if (!hb.fail[next]) break;
+    if (int rc = grow_bins(E, a, i, std::max(4 * B.room[i], next_pow2(hb.rows + hb.rows / 8)), W)) return rc;
+    clear(next);
+    cudaMemcpyAsync(S.bin_state, &hb, sizeof hb, cudaMemcpyHostToDevice, E->stream);
+    if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "binned sweep");
+  }
+  clear(set);
+  hb.phase += 1;
+  hb.bins = to.bins;
+  hb.stride = to.stride;
+  hb.cap = to.cap;
+  hb.grow = 1.0f + 0.5f * (g - 1.0f);
+  a.phase0 = hb.phase;
+  a.dealt_op = hb.op;
+  cudaMemcpyAsync(S.bin_state, &hb, sizeof hb, cudaMemcpyHostToDevice, E->stream);
+  if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "binned sweep");
+  return PQ_OK;
 }
 
 // Runs every op of a plan on the binned sweep: one block alone while the rows
@@ -1688,9 +1751,10 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     }
     // The buffer the stopped window was filling (or the dense rows) is grown.
     const u32 fill = hb.dense_start ? 0 : hb.phase + 1;
-    if (!hb.dense_start && hb.dense_end) {
+    const bool deal = hb.stopped == pq::STOP_DEAL;
+    if (!deal && !hb.dense_start && hb.dense_end) {
       if (int rc = E->ensure_dense(S, next_pow2(std::max<u64>(hb.n_dense, S.cap + 1)), 0, W)) return rc;
-    } else {
+    } else if (!deal) {
       const int i = (int)(fill & 1);
       const u64 have = B.room[i];
       // the rows of the bins the window had finished when it stopped, for all
@@ -1698,15 +1762,9 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
       const u32 tickets = hb.ticket[hb.phase % 3] & (pq::NO_MORE_BINS - 1);
       double need = hb.dense_start ? 0.0 : (double)hb.n[(hb.phase + 1) % 3];
       if (tickets > (u32)grid && tickets - grid < hb.bins) need *= (double)hb.bins / (tickets - grid);
-      u64 want = std::max<u64>(4 * have, next_pow2(4 * hb.rows));
-      want = std::max(want, next_pow2((u64)std::min(1.125 * need, 2.0 * MAX_ROWS)));
-      int rc = E->ensure_bins(B, i, want, W);
-      while (rc == PQ_ERR_OOM && want > 2 * have) rc = E->ensure_bins(B, i, want = std::max(want / 2, 2 * have), W);
-      if (rc == PQ_ERR_OOM && a.spill_limit) {  // as large as it gets: rows may spill as far as there are tags
-        a.spill_limit = 0;
-        rc = E->ensure_bins(B, i, have, W);
-      }
-      if (rc) return rc;
+      const u64 want = std::max<u64>(4 * have, next_pow2(4 * hb.rows));
+      if (int rc = grow_bins(E, a, i, std::max(want, next_pow2((u64)std::min(1.125 * need, 2.0 * MAX_ROWS))), W))
+        return rc;
     }
     // Everything the stopped window counted is dropped.
     for (u32 s = 0; s < 3; ++s) {
@@ -1728,6 +1786,8 @@ int execute_bins(pq_engine* E, Slot& S, Plan& P, bool* began) {
     }
     cudaMemcpyAsync(S.bin_state, &hb, sizeof hb, cudaMemcpyHostToDevice, E->stream);
     if ((e = cudaStreamSynchronize(E->stream)) != cudaSuccess) return E->cuda_fail(e, "binned sweep");
+    if (deal)
+      if (int rc = deal_bins(E, S, P, a, hb, grid)) return rc;
   }
 }
 

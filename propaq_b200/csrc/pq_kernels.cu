@@ -1378,7 +1378,7 @@ __global__ void __launch_bounds__(BLOCK, 2) sweep_kernel_two(const SweepArgs a) 
 // bins, more of them split).
 template <int W>
 struct BinSize {
-  static constexpr int T = 256;
+  static constexpr int T = BIN_THREADS;
   static constexpr int BLOCKS = 2;  // per SM
   static constexpr int GRID_R = W == 1 ? 3328 : (W == 2 ? 2560 : (W == 4 ? 2048 : 1152));
   static constexpr int WARP_R = W <= 4 ? 128 : 120;
@@ -1423,6 +1423,14 @@ __global__ void __launch_bounds__(BinSize<W>::T, BinSize<W>::BLOCKS) bins_kernel
   extern __shared__ __align__(16) unsigned char bin_smem[];
   auto& s = *reinterpret_cast<typename BinSize<W>::GridSmem*>(bin_smem);
   bins_body<W, ALG>(a, Grp{blockIdx.x, gridDim.x}, s.win, s.rows.block, s.rows.warp);
+}
+
+template <int W, int ALG>
+__global__ void __launch_bounds__(BinSize<W>::T) deal_kernel(const __grid_constant__ BinArgs a, u32 win, u32 fill,
+                                                            const __grid_constant__ Layout from,
+                                                            const __grid_constant__ Layout to) {
+  __shared__ WinSmem<W> v;
+  deal_body<W, ALG, BinSize<W>::T>(a, v, win, fill, from, to);
 }
 
 // A batch: each instance owns the contiguous blocks [blk_begin, blk_begin +
@@ -1872,6 +1880,17 @@ cudaError_t launch_bins(const BinArgs& a, int grid, cudaStream_t s) {
 }
 
 template <int W, int ALG>
+cudaError_t launch_deal(const BinArgs& a, u32 win, u32 fill, const Layout& from, const Layout& to, int grid,
+                        cudaStream_t s) {
+  deal_kernel<W, ALG><<<4 * grid, BinSize<W>::T, 0, s>>>(a, win, fill, from, to);
+  return cudaGetLastError();
+}
+template <int W>
+u32 bin_rows() {
+  return BinSize<W>::GRID_R;
+}
+
+template <int W, int ALG>
 cudaError_t launch_batch_sweep(const SweepArgs* args, const u32* block_inst, int grid, cudaStream_t s) {
   void* params[] = {(void*)&args, (void*)&block_inst};
   return cudaLaunchCooperativeKernel((const void*)batch_sweep_kernel<W, ALG>, dim3(grid), dim3(BLOCK), params, 0,
@@ -1953,7 +1972,9 @@ cudaError_t launch_conjugate(const u64* keys, const double* coeffs, u64 n, const
   template int bins_grid<Wv, Av>();                                                                     \
   template cudaError_t launch_solo<Wv, Av>(const BinArgs&, cudaStream_t);                               \
   template cudaError_t launch_solo_batch<Wv, Av>(const BinArgs*, int, cudaStream_t);                     \
-  template cudaError_t launch_bins<Wv, Av>(const BinArgs&, int, cudaStream_t);
+  template cudaError_t launch_bins<Wv, Av>(const BinArgs&, int, cudaStream_t);                          \
+  template cudaError_t launch_deal<Wv, Av>(const BinArgs&, u32, u32, const Layout&, const Layout&, int,  \
+                                           cudaStream_t);
 #define PQ_INSTANTIATE_KEYS(Wv)                                                                         \
   template cudaError_t launch_rebuild<Wv>(const u64*, u64, u64*, u64, u64, u32*, cudaStream_t);         \
   template cudaError_t launch_conjugate<Wv>(const u64*, const double*, u64, const u64*, const int*, u32, int, \
@@ -1979,6 +2000,7 @@ PQ_INSTANTIATE_W(PQ_ONLY_WIDTH)
 #if PQ_ONLY_WIDTH <= 8
 PQ_INSTANTIATE_BINS(PQ_ONLY_WIDTH, 0)
 PQ_INSTANTIATE_BINS(PQ_ONLY_WIDTH, 1)
+template u32 bin_rows<PQ_ONLY_WIDTH>();
 #endif
 #else
 PQ_INSTANTIATE_W(1)
@@ -1987,6 +2009,8 @@ PQ_INSTANTIATE_BINS(1, 0)
 PQ_INSTANTIATE_BINS(1, 1)
 PQ_INSTANTIATE_BINS(2, 0)
 PQ_INSTANTIATE_BINS(2, 1)
+template u32 bin_rows<1>();
+template u32 bin_rows<2>();
 #endif
 
 }  // namespace pq

@@ -182,6 +182,8 @@ struct BasisDesc {
 
 constexpr u32 NO_MORE_BINS = 1u << 30;  // added to a set's ticket when the buffer being filled is too small
 
+enum : u32 { STOP_GROW = 1, STOP_DEAL = 2 };
+
 // Device state of a binned sweep; the sets are indexed by window count mod 3.
 struct BinState {
   u64 n[3];        // rows in the set's bins
@@ -190,7 +192,8 @@ struct BinState {
   u32 n_spill[3];  // rows past a full bin
   u32 ticket[3];   // bins handed out
   u32 fail[3];     // the set's buffer was too small
-  // Where a sweep stopped for a buffer the host has to grow.
+  // Where a sweep stopped: STOP_GROW for a buffer the host has to grow, STOP_DEAL
+  // for rows that need other bins.
   u32 stopped, dense_start;  // dense_start: before any row was dealt
   u32 dense_end, pad_;       // the buffer is the dense rows the last window writes
   u32 op, phase;   // first op not run; count of buffer fills so far
@@ -225,6 +228,7 @@ struct BinArgs {
   u32 count_words;
   u32 spill_limit;    // a buffer with more spills than spill_limit() counts as too small
   u32 resume, phase0; // continue a stopped sweep from BinState
+  u32 dealt_op;       // the op whose rows were dealt again last
   float* growth;      // per window: growth of the live count inside it, rows leaving / entering,
                       // rows entering (0: not run on the grid)
   u32* born;          // per op: rows created
@@ -248,6 +252,14 @@ template <int W, int ALG>
 cudaError_t launch_solo_batch(const BinArgs* args, int n, cudaStream_t s);
 template <int W, int ALG>
 cudaError_t launch_bins(const BinArgs& a, int grid, cudaStream_t s);
+// The rows of a stopped sweep's bins (fill number `fill`) into the bins `to` of
+// the next fill, for window `win`.
+template <int W, int ALG>
+cudaError_t launch_deal(const BinArgs& a, u32 win, u32 fill, const Layout& from, const Layout& to, int grid,
+                        cudaStream_t s);
+// Rows a block of the grid holds.
+template <int W>
+u32 bin_rows();
 
 enum : u32 { LOG_HELD = 0, LOG_L1 = 1, LOG_MAX = 2, LOG_EMITTED = 3, LOG_HITS = 4, LOG_WORDS = 5 };
 
