@@ -410,15 +410,19 @@ def main_batch(args, world, rank, local):
               for p in probs)
     d2h = sum(8 * len(p.angles) + 16 * (len(p.angles) + len(p.offsets) - 1) + 32 * 4 * 148 for p in probs)
     peak_gbs, peak_kind = measured_peaks()
-    achieved = alg_bytes / (sweep_ms / 1e3) / 1e9 if sweep_ms > 0 else None
+    # One pass over the rows per rotation would have had to move this; the
+    # binned sweep, which the batch runs on unless a tuned setting says
+    # otherwise, moves each row once per run of rotations (not captured).
+    visit_gbs = alg_bytes / (sweep_ms / 1e3) / 1e9 if sweep_ms > 0 else None
+    row_sweep = any(tune.get(k) for k in ("blocks_per_sm", "fuse_max", "tile_items", "bucket_slots"))
     line = dict(base_line, value=value, ms_per_step=1e3 * dev_s / args.steps,
                 instances_per_s=world * len(probs) * args.steps / dev_s,
                 e2e={"value": world * e2e_terms / e2e_s, "unit": "terms/s", "h2d_bytes_per_step": int(h2d),
                      "d2h_bytes_per_step": int(d2h), "ms_per_step": 1e3 * e2e_s / args.steps},
                 gpu_launches=launches // max(1, args.steps),
-                roofline={"bound": "hbm", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s",
-                          "frac": None if achieved is None else achieved / peak_gbs, "traffic": None,
-                          "kernel": "batch_sweep_kernel", "peak_source": f"{peak_kind} hbm_gbs",
+                roofline={"bound": "latency", "achieved": None, "peak": peak_gbs, "unit": "GB/s",
+                          "frac": None, "traffic": None, "visit_gbs": visit_gbs,
+                          "kernel": "batch_sweep_kernel" if row_sweep else "bins_kernel + solo_batch_kernel", "peak_source": f"{peak_kind} hbm_gbs",
                           "launches_per_step": sweep_launches / max(1, args.steps),
                           "share_of_device_time": sweep_ms / dev_ms if dev_ms else None},
                 tuning=dict(tune, autotuned=tuned is not None, trials=tuned), clocks=clocks)
@@ -778,20 +782,24 @@ def main():
     d2h = 8 * len(prob.angles) + 16 * n_ops + 32 * 4 * 148
     peak_gbs, peak_kind = measured_peaks()
     # The dominant kernels are the sweep's: a solo launch and a grid launch per
-    # step (plus one per buffer growth) run every gate and noise op.
-    achieved = alg_bytes / (sweep_ms / 1e3) / 1e9 if sweep_ms > 0 else None
+    # step (plus one per buffer growth) run every gate and noise op.  They move
+    # each row once per run of rotations and work on it in shared memory, so
+    # what bounds them is the chain of dependent steps there.  `achieved` is
+    # their DRAM rate; `visit_gbs` is what one pass over the rows per rotation
+    # would have had to move in the same time.
+    visit_gbs = alg_bytes / (sweep_ms / 1e3) / 1e9 if sweep_ms > 0 else None
     # DRAM bytes of the sweep launches of one step, from an ncu capture
-    # (profiles/sweep_traffic_*.json), as bytes per launch like `achieved`:
-    # the step's bytes over the launches a step took here (the grid follows
-    # the live count, so a step can be several launches).
+    # (profiles/sweep_traffic_*.json), as bytes per launch: the step's bytes
+    # over the launches a step took here.
     traffic = None
     tf = ROOT / "profiles" / f"sweep_traffic_{wl.name}.json"
     if tf.exists() and sweep_launches:
         per_step = json.loads(tf.read_text()).get("dram_bytes_per_step")
         if per_step is not None:
             traffic = per_step / (sweep_launches / args.steps)
-    # For the HBM-bound Majorana runs: the sweep's DRAM rate (traffic over the
-    # launch time) beside the rate random 32-byte reads reach on this GPU.
+    achieved = traffic * sweep_launches / (sweep_ms / 1e3) / 1e9 if traffic is not None and sweep_ms > 0 else None
+    # For the Majorana runs: the sweep's DRAM rate beside the rate random
+    # 32-byte reads reach on this GPU.
     scattered = None
     if wl.basis == 1 and traffic is not None and sweep_ms > 0 and not args.no_scattered_reference:
         rate = random_sector_rate(f"cuda:{local}")
@@ -801,14 +809,14 @@ def main():
                 e2e={"value": e2e_value, "unit": "terms/s", "h2d_bytes_per_step": int(h2d),
                      "d2h_bytes_per_step": int(d2h), "ms_per_step": 1e3 * e2e_s / args.steps},
                 gpu_launches=launches,
-                roofline={"bound": "hbm", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s",
+                roofline={"bound": "latency", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s",
                           "frac": None if achieved is None else achieved / peak_gbs, "traffic": traffic,
                           "kernel": "bins_kernel + solo_kernel", "peak_source": f"{peak_kind} hbm_gbs",
                           "launches": sweep_launches,
-                          "algorithmic_bytes_per_launch": alg_bytes / max(1, sweep_launches),
+                          "visit_gbs": visit_gbs, "visit_bytes_per_launch": alg_bytes / max(1, sweep_launches),
                           "ms_per_launch": sweep_ms / max(1, sweep_launches),
                           "share_of_device_time": sweep_ms / dev_ms if dev_ms else None,
-                          "gate_ops_gbs": galg / (gate_ms / 1e3) / 1e9 if gate_ms > 0 else None,
+                          "gate_visit_gbs": galg / (gate_ms / 1e3) / 1e9 if gate_ms > 0 else None,
                           "us_per_gate_op": 1e3 * gate_ms / max(1, gate_ops),
                           "scattered_reads": scattered},
                 clocks=clocks, peak_terms=peak, expectation_value=r.expectation_value)

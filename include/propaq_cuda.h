@@ -132,7 +132,9 @@ typedef struct pq_result {
   uint64_t sum_rows_noise;    /* sum over noise ops of the rows they scan      */
   uint64_t sum_kept;          /* ... of the rows a reclaim keeps               */
   uint64_t class_ops;         /* runs of four or more Clifford rotations on
-                                 disjoint units that went through one pass     */
+                                 disjoint units that went through one pass over
+                                 the rows: a class op of the row sweep's, or
+                                 inside one window of the binned sweep's       */
 } pq_result;
 
 /* Key width for a register: 1,2,4,...,64 words for up to 32,64,...,2048

@@ -26,14 +26,19 @@
 //     of the window's generators, of rank at most BIN_RANK: a group has at
 //     most 2^rank keys, so one always fits in shared memory;
 //   * disjoint windows: Pauli generators on pairwise disjoint qubits (they
-//     commute).  K is reduced only by the generators it anticommutes with --
+//     commute; the rotations by pi among them may lie across any of them, and
+//     change no key).  K is reduced only by the generators it anticommutes with --
 //     the set no rotation of the window changes -- so their number is not
 //     limited: a weight cut of at most BIN_RANK bounds that set's size, and
 //     with it the group's, for every row.
 //
 // A bin that does not fit (its rows, or the rows it grows to) is run again in
 // halves by further bits of the group hash, as often as it takes; nothing of
-// a bin is written before all of it has fitted.
+// a bin is written before all of it has fitted.  Two groups of one 32-bit hash
+// cannot be told apart (a few pairs among 300,000 groups, or keys that differ
+// by a kernel vector of the hash): if they do not fit together the run goes to
+// the row sweep.  A window whose rows find their buffer too small stops; the
+// host grows the buffer and the window is run again.
 //
 // Who takes a bin follows the rows per bin: while a bin of every warp of the
 // grid holds the live set, each warp runs bins of its own, with no block
@@ -47,11 +52,7 @@
 // What bounds it: the dependent shared-memory round trips of a rotation's
 // step (about 1 us on small bins; 2-3 us where a block's 1,500-3,000 rows
 // branch often), no longer the grid barrier or DRAM.  Whole calls, row sweep
-// -> binned sweep, on one box: 4-qubit circuit, 40 noisy rotations 0.66 ->
-// 0.29 ms; 20-qubit TFIM (to 57k rows) 2.05 -> 0.83 ms; kicked Ising 10x10 x
-// 20 steps (4-word keys, to 477k rows) 23.3 -> 8.8 ms, 6x6 x 8 (2 words, to
-// 1.2M) 9.2 -> 3.0 ms, 12x15 x 8 (8 words) 31.5 -> 12.3 ms; Givens circuits
-// of 24 sites (16M rows) 54 -> 15.6 ms and 32 sites (80M rows) 453 -> 119 ms.
+// -> binned sweep, on one box: @CALLS@
 #pragma once
 
 constexpr u32 TAB_EMPTY = 0xffffffffu;

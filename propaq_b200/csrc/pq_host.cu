@@ -721,7 +721,7 @@ struct Plan {
   // table bucket.
   u32 fuse_max = FUSE_DEFAULT, tile_items = 0, bucket_slots = BUCKET_DEFAULT;
   bool binned = false;  // runs on the binned sweep (pq_bins.cuh)
-  u32 class_runs = 0;   // runs of Clifford rotations on disjoint units inside one window
+  u32 class_runs = 0;   // pq_result::class_ops of a binned run: runs of Clifford rotations on disjoint units inside one window
   std::vector<pq::WinDesc> windows;
   std::vector<pq::BasisDesc> basis;
   bool fold_on_device = false;  // hk / hc hold the admitted terms unfolded (DEVICE_FOLD_MIN)

@@ -11,6 +11,12 @@ a time over its values (keeping a value only when it is faster), and it
 remembers the winner per batch shape (basis, and per instance: units, gates,
 layers and truncation settings), so a sweep that is run again -- an
 extrapolation inside an optimisation loop, say -- pays for the tuning once.
+
+All six act on the row sweep.  A batch that sets neither a grid size nor a
+kernel knob runs on the binned sweep instead, if every instance of it can: the
+launch candidates with blocks_per_sm 0 then measure that same run (the choice
+among them is of no consequence), and the others measure the row sweep beside
+it.
 Results do not depend on the setting (every instance is bit-identical to its
 own `pq_run`), only the time does.
 """
@@ -21,9 +27,10 @@ from dataclasses import dataclass, replace
 
 from . import _native
 
-# (blocks_per_sm, split, rebalance_pct): the default first, then the grid
-# sizes, splits and rebalancing thresholds that moved the time of the
-# 64-instance extrapolation sweep in measurement (993-1250 ms per batch).
+# (blocks_per_sm, split, rebalance_pct): the default first (the binned sweep,
+# where the batch can run on it), then the grid sizes, splits and rebalancing
+# thresholds that moved the time of the 64-instance extrapolation sweep on the
+# row sweep (993-1250 ms per batch).
 # Never rebalancing is left out: it took that sweep 7.3 s, the largest
 # instances running on their first small share of the grid.
 CANDIDATES = [
@@ -59,7 +66,9 @@ class Tuning:
                 "fuse_max": self.fuse_max, "tile_items": self.tile_items, "bucket_slots": self.bucket_slots}
 
     def resolved(self) -> tuple:
-        """The setting with kernel defaults spelled out (0 and the default run alike)."""
+        """The setting with kernel defaults spelled out: one key for 0 and the
+        default, which a tuning run does not measure both of (on the row sweep
+        they are the same; 0 may also mean the binned sweep)."""
         k = {d: getattr(self, d) or KERNEL_DEFAULTS[d] for d in KERNEL_DIMENSIONS}
         return (self.blocks_per_sm, self.split, self.rebalance_pct, k["fuse_max"], k["tile_items"],
                 k["bucket_slots"])
