@@ -2033,7 +2033,7 @@ int finalize(pq_engine* E, Slot& S, Plan& P, std::vector<pq::ExpectPartial>* par
         u64* sk = scratch + sw;
         double* sc = reinterpret_cast<double*>(sk + n_fin * W);
         e = with_words(W, [&](auto w) {
-          return pq::sort_rows<decltype(w)::value>(out_k, out_c, n_fin, sk, sc, scratch, E->stream, &E->launches);
+          return pq::sort_rows<decltype(w)::value>(out_k, out_c, n_fin, sk, sc, scratch, E->stream, &E->launches, true);
         });
         if (e != cudaSuccess) return E->cuda_fail(e, "sorting the terms");
         out_k = sk;

@@ -37,8 +37,13 @@ namespace pq {
 namespace {
 
 constexpr int SORT_BLOCK = 256;
-constexpr int SORT_CHUNKS = 8;                       // 256-row chunks per tile
-constexpr int SORT_TILE = SORT_BLOCK * SORT_CHUNKS;  // rows per block per pass
+// 256-row chunks per tile, one block's rows of a pass: few rows are spread over
+// more blocks (20,000 rows in tiles of 2,048 are 10 blocks).
+inline int sort_chunks(u64 n) { return n <= (1u << 17) ? 1 : 8; }
+inline u64 sort_blocks(u64 n) {
+  const u64 tile = (u64)SORT_BLOCK * sort_chunks(n);
+  return (n + tile - 1) / tile;
+}
 constexpr int SORT_WARPS = SORT_BLOCK / 32;
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
@@ -66,12 +71,12 @@ __global__ void __launch_bounds__(SORT_BLOCK) digit_tally_kernel(const u64* keys
 
 template <int W>
 __global__ void __launch_bounds__(SORT_BLOCK) digit_count_kernel(const u64* keys, u64 n, int pass, u32* counts,
-                                                                 u32 nblk) {
+                                                                 u32 nblk, int chunks) {
   __shared__ u32 c[256];
   c[threadIdx.x] = 0;
   __syncthreads();
-  const u64 base = (u64)blockIdx.x * SORT_TILE;
-  for (int i = 0; i < SORT_CHUNKS; ++i) {
+  const u64 base = (u64)blockIdx.x * SORT_BLOCK * chunks;
+  for (int i = 0; i < chunks; ++i) {
     const u64 r = base + (u64)i * SORT_BLOCK + threadIdx.x;
     if (r < n) atomicAdd(&c[digit_of<W>(keys, r, pass)], 1u);
   }
@@ -144,7 +149,7 @@ __global__ void __launch_bounds__(T) digit_scan_kernel(u32* counts, u32 nblk, co
 
 template <int W>
 __global__ void __launch_bounds__(SORT_BLOCK) digit_scatter_kernel(const u64* keys, const double* coeffs, u64 n,
-                                                                   int pass, const u32* offsets, u32 nblk,
+                                                                   int pass, const u32* offsets, u32 nblk, int chunks,
                                                                    u64* keys_out, double* coeffs_out) {
   __shared__ u32 run[256];                // next output place of each digit for this block
   __shared__ u32 wcnt[SORT_WARPS][256];   // rows of each digit in each warp of the chunk
@@ -152,8 +157,8 @@ __global__ void __launch_bounds__(SORT_BLOCK) digit_scatter_kernel(const u64* ke
   run[threadIdx.x] = offsets[(u64)threadIdx.x * nblk + blockIdx.x];
   for (int w = 0; w < SORT_WARPS; ++w) wcnt[w][threadIdx.x] = 0;
   __syncthreads();
-  const u64 base = (u64)blockIdx.x * SORT_TILE;
-  for (int i = 0; i < SORT_CHUNKS; ++i) {
+  const u64 base = (u64)blockIdx.x * SORT_BLOCK * chunks;
+  for (int i = 0; i < chunks; ++i) {
     const u64 r = base + (u64)i * SORT_BLOCK + threadIdx.x;
     const bool live = r < n;
     const u32 d = live ? digit_of<W>(keys, r, pass) : 256u + (u32)lane;  // dead lanes match nobody
@@ -177,6 +182,42 @@ __global__ void __launch_bounds__(SORT_BLOCK) digit_scatter_kernel(const u64* ke
     run[threadIdx.x] += add;
     __syncthreads();
   }
+}
+
+// Few rows, distinct keys: a row's place is the number of smaller keys, counted
+// against all of them, tile by tile in shared memory.  n^2 comparisons in one
+// launch where the radix passes are up to 24 W launches and a read-back: 87
+// rows of 8 words 1.1 -> 0.05 ms, 1,797 of them 1.7 -> 0.13, 12,284 2.3 -> 0.8,
+// 5,163 rows of 1 word 0.16 -> 0.10.
+constexpr int RANK_LANES = 8;  // that share a row's comparisons
+constexpr int RANK_T = 256, RANK_BLOCK_ROWS = RANK_T / RANK_LANES;
+template <int W>
+__global__ void __launch_bounds__(RANK_T) rank_sort_kernel(const u64* keys, const double* coeffs, u32 n, u64* keys_out,
+                                                           double* coeffs_out) {
+  __shared__ u64 tile[RANK_T][W + 1];  // one more: the lanes of a row read rows of different banks
+  const u32 r = blockIdx.x * RANK_BLOCK_ROWS + threadIdx.x / RANK_LANES, lane = threadIdx.x % RANK_LANES;
+  u64 k[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) k[w] = r < n ? keys[(u64)r * W + w] : 0;
+  u32 place = 0;
+  for (u32 t0 = 0; t0 < n; t0 += RANK_T) {
+    const u32 m = n - t0 < (u32)RANK_T ? n - t0 : (u32)RANK_T;
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < m * W; i += RANK_T) tile[i / W][i % W] = keys[(u64)t0 * W + i];
+    __syncthreads();
+    for (u32 j = lane; j < m; j += RANK_LANES) {
+      bool less = false;
+#pragma unroll
+      for (int w = 0; w < W; ++w) less = tile[j][w] < k[w] || (tile[j][w] == k[w] && less);
+      place += less ? 1u : 0u;
+    }
+  }
+#pragma unroll
+  for (int o = RANK_LANES / 2; o > 0; o >>= 1) place += __shfl_xor_sync(FULL_MASK, place, o);
+  if (r >= n || lane) return;
+#pragma unroll
+  for (int w = 0; w < W; ++w) keys_out[(u64)place * W + w] = k[w];
+  coeffs_out[place] = coeffs[r];
 }
 
 // 1 where a sorted row starts a run of equal keys.
@@ -215,15 +256,24 @@ inline int grid_for(u64 n, int block) {
 }  // namespace
 
 u64 sort_scratch_words(u64 n, int W) {
-  const u64 nblk = (n + SORT_TILE - 1) / SORT_TILE;
+  const u64 nblk = sort_blocks(n);
   return 256 * (nblk ? nblk : 1) / 2 + 1 + (u64)8 * W * 256 / 2 + n * (u64)W + n;
 }
 
 template <int W>
 cudaError_t sort_rows(const u64* keys, const double* coeffs, u64 n, u64* keys_out, double* coeffs_out,
-                      u64* scratch, cudaStream_t s, u64* launches) {
+                      u64* scratch, cudaStream_t s, u64* launches, bool distinct) {
   if (n == 0) return cudaSuccess;
-  const u32 nblk = (u32)((n + SORT_TILE - 1) / SORT_TILE);
+  if constexpr (W <= 8) {
+    if (distinct && n <= RANK_ROWS) {
+      rank_sort_kernel<W><<<(u32)((n + RANK_BLOCK_ROWS - 1) / RANK_BLOCK_ROWS), RANK_T, 0, s>>>(keys, coeffs, (u32)n,
+                                                                                            keys_out, coeffs_out);
+      ++*launches;
+      return cudaGetLastError();
+    }
+  }
+  const u32 nblk = (u32)sort_blocks(n);
+  const int chunks = sort_chunks(n);
   const u64 m = 256ull * nblk;
   // scratch: counts (m u32), tally (8W x 256 u32), then a second key / coefficient buffer
   u32* counts = reinterpret_cast<u32*>(scratch);
@@ -255,10 +305,10 @@ cudaError_t sort_rows(const u64* keys, const double* coeffs, u64 n, u64* keys_ou
     const bool to_out = ((np - 1 - i) & 1) == 0;
     u64* dk = to_out ? keys_out : tk;
     double* dc = to_out ? coeffs_out : tc;
-    digit_count_kernel<W><<<nblk, SORT_BLOCK, 0, s>>>(src_k, n, passes[i], counts, nblk);
+    digit_count_kernel<W><<<nblk, SORT_BLOCK, 0, s>>>(src_k, n, passes[i], counts, nblk, chunks);
     if (nblk <= 1024) digit_scan_kernel<256><<<256, 256, 0, s>>>(counts, nblk, tally + passes[i] * 256);
     else digit_scan_kernel<1024><<<256, 1024, 0, s>>>(counts, nblk, tally + passes[i] * 256);
-    digit_scatter_kernel<W><<<nblk, SORT_BLOCK, 0, s>>>(src_k, src_c, n, passes[i], counts, nblk, dk, dc);
+    digit_scatter_kernel<W><<<nblk, SORT_BLOCK, 0, s>>>(src_k, src_c, n, passes[i], counts, nblk, chunks, dk, dc);
     *launches += 3;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     src_k = dk;
@@ -296,7 +346,8 @@ cudaError_t fold_sorted(const u64* keys, const double* coeffs, u64 n, u64* keys_
 }
 
 #define PQ_SORT_INSTANTIATE(Wv)                                                                                  \
-  template cudaError_t sort_rows<Wv>(const u64*, const double*, u64, u64*, double*, u64*, cudaStream_t, u64*); \
+  template cudaError_t sort_rows<Wv>(const u64*, const double*, u64, u64*, double*, u64*, cudaStream_t, u64*,  \
+                                     bool);                                                                     \
   template cudaError_t fold_sorted<Wv>(const u64*, const double*, u64, u64*, double*, u32*, u64*, u64*,         \
                                        cudaStream_t, u64*);
 PQ_SORT_INSTANTIATE(1)
