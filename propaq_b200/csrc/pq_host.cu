@@ -1271,7 +1271,14 @@ bool use_bins(const pq_engine* E, const Plan& P) {
 void plan_windows(Plan& P) {
   const int W = P.W;
   const size_t gw = gdesc_words(W), no = P.ops.size();
-  const u32 rank_max = pq::bin_rank(W);
+  // A register of few units can fill its whole key space, 2^(2 n) keys.  Groups
+  // of 2^11 rows are then too few for the blocks and pack badly into them: 9
+  // sites, 262,143 live rows, 159 rotations took 7.7 ms where the row sweep takes
+  // 2.1, and 1.0 with groups of 2^7; 12 qubits, 7.8M rows, 6.9, 4.1 and 3.0 (2^8).
+  // From 2^26 keys on live sets are sparse, and longer windows pay (20-qubit
+  // TFIM 0.46 ms at 2^11, 0.52 at 2^10).
+  const u32 key_bits = 2 * P.n_units;
+  const u32 rank_max = key_bits > 11 && key_bits <= 24 ? std::min(pq::bin_rank(W), 4 + key_bits / 5) : pq::bin_rank(W);
   auto is_rot = [&](size_t i) { return P.ops[i].kind == pq::OP_GATE || P.ops[i].kind == pq::OP_PHASE; };
   auto gen = [&](size_t i) { return &P.gdesc[P.ops[i].idx * gw]; };
   auto lowest = [&](const u64* g) {
@@ -1280,7 +1287,7 @@ void plan_windows(Plan& P) {
     return -1;
   };
   auto bit = [](const u64* g, int b) { return (g[b >> 6] >> (b & 63)) & 1; };
-  const bool disjoint_ok = P.alg == 0 && P.has_w && P.wcut <= rank_max;
+  const bool disjoint_ok = P.alg == 0 && P.has_w && P.wcut <= pq::bin_rank(W);
   std::vector<std::vector<u64>> span;
   std::vector<int> pivot;
   std::vector<u64> used(W), g(W);

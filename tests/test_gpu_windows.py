@@ -10,7 +10,8 @@ every coefficient bit for bit, expectation value.
 * Groups that the 32-bit group hash cannot tell apart and that one block cannot
   hold together: the run takes the row sweep.
 * Windows that multiply their rows by up to 2^11, so that the next window's
-  bins, laid out before, hold many times too few."""
+  bins, laid out before, hold many times too few.
+* Registers so small that their live set fills the key space."""
 
 from __future__ import annotations
 
@@ -21,8 +22,8 @@ import pytest
 from harness import (assert_terms_equal, expectation_close, from_circuit, make_cfg, run_gpu, run_gpu_batch, run_oracle)
 
 from propaq_b200 import _native
-from propaq_b200.circuits import PauliCircuit, PauliRotation
-from propaq_b200.datatypes import PauliString, PauliTermSum
+from propaq_b200.circuits import MajoranaCircuit, MajoranaRotation, PauliCircuit, PauliRotation
+from propaq_b200.datatypes import MajoranaMonomial, MajoranaTermSum, PauliString, PauliTermSum
 
 
 def check(g, o):
@@ -192,3 +193,49 @@ def test_windows_that_multiply_their_rows(k, n, width, pairs):
     for r in (binned, row):
         assert abs(r.expectation_value - want) <= 1e-12 * float(np.sum(np.abs(p.obs_coeffs)))
     assert binned.device_ms < 3.0 * row.device_ms
+
+
+# --------------------------------------------------------- small registers
+def full_majorana(sites, n_gates):
+    rng = np.random.default_rng(sites)
+    m = 2 * sites
+    rots = []
+    for _ in range(n_gates):
+        modes = rng.choice(m, size=int(rng.integers(1, 5)), replace=False)
+        rots.append(MajoranaRotation(MajoranaMonomial(sum(1 << int(v) for v in modes), m, False),
+                                     float(rng.uniform(-1, 1))))
+    obs = MajoranaTermSum()
+    obs.add(MajoranaMonomial(3, m), 1.0)
+    return from_circuit(1, sites, obs, MajoranaCircuit([rots]), 5)
+
+
+def full_pauli(n, n_gates):
+    rng = np.random.default_rng(n)
+    rots = []
+    for _ in range(n_gates):
+        x = z = 0
+        for q in rng.choice(n, size=min(n, int(rng.integers(1, 4))), replace=False):
+            t = int(rng.integers(1, 4))
+            x |= (t & 1) << int(q)
+            z |= (t >> 1) << int(q)
+        rots.append(PauliRotation(PauliString(x, z, n), float(rng.uniform(-1.2, 1.2))))
+    return from_circuit(0, n, PauliTermSum({PauliString(0, 1, n): 1.0}), PauliCircuit([rots]), 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [lambda: full_majorana(7, 90), lambda: full_majorana(9, 130), lambda: full_pauli(5, 60),
+                                  lambda: full_pauli(6, 60), lambda: full_pauli(9, 90)],
+                         ids=["7 sites", "9 sites", "5 qubits", "6 qubits", "9 qubits"])
+def test_live_sets_that_fill_the_key_space(gpu_engine, oracle, make):
+    p = make()
+    g = run_gpu(gpu_engine, p)
+    check(g, run_oracle(oracle, p))
+    assert g.n_final > (1 << (2 * p.n_units)) // 4
+    # and not slower than a pass per rotation by much (9 sites: 0.7-1.2 ms
+    # against 1.4-2.2; 2.2-7.7 with windows as long as on wide registers)
+    cfg, keep = make_cfg(p, want_terms=False)
+    times = []
+    for knob in (0, 0, 2, 2):
+        cfg.fuse_max = knob
+        times.append(gpu_engine.run(cfg, p.obs_keys, p.obs_coeffs, p.gate_keys, p.angles, p.offsets, p.diag)[0].device_ms)
+    assert times[1] < 1.5 * times[3]
