@@ -119,7 +119,8 @@ typedef struct pq_result {
   double sweep_ms;            /* CUDA-event time of the sweep kernel launches  */
   uint64_t sweep_launches;    /* row sweep: 1, plus one per capacity growth and
                                  per larger grid; binned sweep: a solo and a grid
-                                 launch, plus one per capacity growth           */
+                                 launch (the grid's left out where one block
+                                 certainly runs it all), plus one per growth    */
   /* Split of the sweep time by op kind: from the device clock at each op's end
    * (row sweep), or at the end of a run of rotations and the noise after it,
    * whose time is shared among its ops by the rows they scan (binned sweep). */

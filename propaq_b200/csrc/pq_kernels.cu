@@ -1385,7 +1385,7 @@ struct BinSize {
   static constexpr int SOLO_WARP_R = 128;  // up to 64 rows: two rounds of 32 at the most
   // solo up to 1,024 rows: beyond, a rotation takes the block 1.5 us and more,
   // a grid window of a dozen rotations 17 us
-  static constexpr int SOLO_R = 2048;
+  static constexpr int SOLO_R = SOLO_ROWS;
   using Warp = BinSmem<W, 32, WARP_R, 512>;
   using Grid = BinSmem<W, T, GRID_R, (W <= 2 ? 8192 : 4096)>;
   using SoloWarp = BinSmem<W, 32, SOLO_WARP_R, 512>;

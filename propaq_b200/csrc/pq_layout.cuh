@@ -7,6 +7,7 @@
 namespace pq {
 
 constexpr u32 BIN_THREADS = 256;   // of a block
+constexpr u32 SOLO_ROWS = 2048;    // of a block alone; a rotation runs while it may double its rows
 constexpr u32 BIN_MAX = 1u << 18;  // bins of one buffer
 constexpr u32 COUNT_WORDS = BIN_MAX;  // words of one counter set (fewer bins, wider stride: choose_layout)
 

@@ -11,7 +11,8 @@ every coefficient bit for bit, expectation value.
   hold together: the run takes the row sweep.
 * Windows that multiply their rows by up to 2^11, so that the next window's
   bins, laid out before, hold many times too few.
-* Registers so small that their live set fills the key space."""
+* Registers so small that their live set fills the key space, and circuits so
+  short that one block certainly runs them."""
 
 from __future__ import annotations
 
@@ -239,3 +240,21 @@ def test_live_sets_that_fill_the_key_space(gpu_engine, oracle, make):
         cfg.fuse_max = knob
         times.append(gpu_engine.run(cfg, p.obs_keys, p.obs_coeffs, p.gate_keys, p.angles, p.offsets, p.diag)[0].device_ms)
     assert times[1] < 1.5 * times[3]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_terms,n_gates", [(1, 0), (1, 1), (1, 11), (1, 12), (511, 2), (512, 2), (513, 2), (1024, 1),
+                                             (1025, 1), (1025, 0)])
+def test_short_circuits(gpu_engine, oracle, n_terms, n_gates):
+    # every rotation doubles every row: on either side of what one block runs
+    n = 24
+    rng = np.random.default_rng(n_terms)
+    x = [PauliRotation(PauliString(1 << q, 0, n), float(rng.uniform(0.3, 1.2))) for q in range(n_gates)]
+    obs = PauliTermSum({PauliString(0, ((1 << 12) - 1) | i << 12, n): float(rng.normal()) for i in range(n_terms)})
+    p = from_circuit(0, n, obs, PauliCircuit([x] if x else []), 0)
+    g = run_gpu(gpu_engine, p)
+    check(g, run_oracle(oracle, p))
+    assert g.n_final == n_terms << n_gates
+    alone = n_gates == 0 or n_terms << (n_gates - 1) <= 1024
+    if alone:
+        assert g.res.sweep_launches == 1
