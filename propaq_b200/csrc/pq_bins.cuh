@@ -23,7 +23,8 @@
 // Group hashes (host: plan_windows).  Keys are hashed by a GF(2)-linear map h
 // (lin_hash), so h(K ^ G) = h(K) ^ h(G) and a child's hash costs one xor.
 //   * span windows: the hash of K reduced by a row-echelon basis of the span
-//     of the window's generators, of rank at most BIN_RANK: a group has at
+//     of the window's generators, of rank at most BIN_RANK (less on registers
+//     whose key space can fill up): a group has at
 //     most 2^rank keys, so one always fits in shared memory;
 //   * disjoint windows: Pauli generators on pairwise disjoint qubits (they
 //     commute; the rotations by pi among them may lie across any of them, and
@@ -52,7 +53,11 @@
 // What bounds it: the dependent shared-memory round trips of a rotation's
 // step (about 1 us on small bins; 2-3 us where a block's 1,500-3,000 rows
 // branch often), no longer the grid barrier or DRAM.  Whole calls, row sweep
-// -> binned sweep, on one box: @CALLS@
+// -> binned sweep, on one box: 4-qubit circuit, 40 noisy rotations 0.68 ->
+// 0.32 ms; 20-qubit TFIM (to 31k rows) 1.8 -> 0.80 ms; kicked Ising 10x10 x 20
+// steps (4-word keys, to 476k rows) 23.6 -> 8.1 ms, 6x6 x 8 (2 words, to over
+// 1M) 9.3 -> 2.7 ms, 12x15 x 8 (8 words) 32 -> 6.3 ms; Givens circuits of 24
+// sites (15M rows) 44 -> 14 ms and 32 sites (99M rows) 428 -> 117 ms.
 #pragma once
 
 constexpr u32 TAB_EMPTY = 0xffffffffu;
