@@ -2154,7 +2154,8 @@ int finish(pq_engine* E, Slot& S, Plan& P, const std::vector<pq::ExpectPartial>&
         if (b == grid_op) from = stamps[no + 1];
         double all = 0;
         for (size_t k = b; k <= i; ++k) all += share(k);
-        for (size_t k = b; k <= i; ++k) op_ms[k] = ms(from, stamps[i]) * share(k) / all;
+        const double unit = ms(from, stamps[i]) / all;
+        for (size_t k = b; k <= i; ++k) op_ms[k] = unit * share(k);
         from = stamps[i];
         b = i + 1;
       }

@@ -183,10 +183,10 @@ def test_windows_that_multiply_their_rows(k, n, width, pairs):
     cfg, keep = make_cfg(p, want_terms=False)
     runs = []
     for knob in (0, 2):
-        cfg.fuse_max = knob
-        for _ in range(2):  # the first one grows the buffers
-            runs.append(engine.run(cfg, p.obs_keys, p.obs_coeffs, p.gate_keys, p.angles, p.offsets, p.diag))
-    (binned, nb), (row, nr) = runs[1], runs[3]
+        cfg.fuse_max = knob  # the first run grows the buffers; the fastest of the others counts
+        several = [engine.run(cfg, p.obs_keys, p.obs_coeffs, p.gate_keys, p.angles, p.offsets, p.diag) for _ in range(4)]
+        runs.append(min(several[1:], key=lambda r: r[0].device_ms))
+    (binned, nb), (row, nr) = runs
     assert np.array_equal(nb, nr) and int(nb[-1]) == 3 ** len(pairs) << (k + n - len(pairs))
     for f in ("n_final", "peak_terms", "sum_anti", "sum_children", "sum_rows_gate"):
         assert getattr(binned, f) == getattr(row, f), f
@@ -235,11 +235,12 @@ def test_live_sets_that_fill_the_key_space(gpu_engine, oracle, make):
     # and not slower than a pass per rotation by much (9 sites: 0.7-1.2 ms
     # against 1.4-2.2; 2.2-7.7 with windows as long as on wide registers)
     cfg, keep = make_cfg(p, want_terms=False)
-    times = []
-    for knob in (0, 0, 2, 2):
+    best = []
+    for knob in (0, 2):
         cfg.fuse_max = knob
-        times.append(gpu_engine.run(cfg, p.obs_keys, p.obs_coeffs, p.gate_keys, p.angles, p.offsets, p.diag)[0].device_ms)
-    assert times[1] < 1.5 * times[3]
+        best.append(min(gpu_engine.run(cfg, p.obs_keys, p.obs_coeffs, p.gate_keys, p.angles, p.offsets, p.diag)[0].device_ms
+                        for _ in range(4)))
+    assert best[0] < 1.5 * best[1]
 
 
 @pytest.mark.gpu
